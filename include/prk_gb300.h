@@ -170,11 +170,11 @@ int prk_gb300_slab_norm(int radius, int64_t n, int dtype, int64_t row_begin, int
  *   start at zero). Calls that overlap on the GPU, e.g. on two streams, race on it. */
 int prk_gb300_norm_noalloc(int radius, int64_t n, int dtype, const void* out, double* norm_dev, void* stream);
 
-/* Process-wide settings. PRK_CFG_KERNEL selects the stencil kernel family: 0 = automatic (for the
- * fused form, the TMA tile kernels on 16-byte-aligned buffers with n a multiple of 2 (FP64) or 4
- * (FP32C) and the plain-staged tile kernels on other shapes; the generic kernels for the form
- * without in_next), 1 = generic kernels only, 2 = TMA kernels required (calls that are not
- * eligible fail with PRK_ERR_ARG). Returns the previous value, or a negative error. Callable from
+/* Process-wide settings. PRK_CFG_KERNEL selects the stencil kernel family: 0 = automatic (the TMA
+ * tile kernels on 16-byte-aligned buffers with n a multiple of 2 (FP64) or 4 (FP32C) and the
+ * plain-staged tile kernels on other shapes, with or without in_next), 1 = generic kernels only,
+ * 2 = TMA kernels required (calls that are not eligible, and those without in_next, fail with
+ * PRK_ERR_ARG). Returns the previous value, or a negative error. Callable from
  * any thread; it governs the calls that start after it returns. */
 #define PRK_CFG_KERNEL 1
 int prk_gb300_config(int key, int value);

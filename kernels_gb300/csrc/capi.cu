@@ -76,6 +76,14 @@ struct DevScratch {
 std::mutex g_scratch_mu;
 std::vector<DevScratch> g_scratch;
 
+// While it lives, the calling thread may allocate although a stream is being captured (its own, or
+// another thread's in the global mode). Allocations are not captured.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 int dev_scratch(DevScratch* out)
 {
     int dev = 0;
@@ -86,6 +94,10 @@ int dev_scratch(DevScratch* out)
     if (g_scratch[dev].norm && ctx != 0 && g_scratch[dev].context != 0 && ctx != g_scratch[dev].context)
         g_scratch[dev] = DevScratch{};  // the old context and its memory are gone
     if (!g_scratch[dev].norm) {
+        // The first call may come while a stream is being captured (the operator form into a caller's
+        // graph), so the scratch is cleared on a stream of its own: the legacy stream would join the
+        // capture.
+        RelaxedCapture relaxed;
         void* p = nullptr;
         const size_t bytes = (prk::NORM_BLOCKS + 1) * sizeof(double) + 256;
         cudaError_t e = cudaMalloc(&p, bytes);
@@ -93,8 +105,15 @@ int dev_scratch(DevScratch* out)
             cudaGetLastError();
             return fail(PRK_ERR_NOMEM, "cudaMalloc of the library scratch failed: %s", cudaGetErrorString(e));
         }
-        e = cudaMemset(p, 0, bytes);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMemset of the library scratch");
+        cudaStream_t clear = nullptr;
+        if ((e = cudaStreamCreateWithFlags(&clear, cudaStreamNonBlocking)) == cudaSuccess) {
+            if ((e = cudaMemsetAsync(p, 0, bytes, clear)) == cudaSuccess) e = cudaStreamSynchronize(clear);
+            cudaStreamDestroy(clear);
+        }
+        if (e != cudaSuccess) {
+            cudaFree(p);
+            return cuda_fail(e, "clearing the library scratch");
+        }
         g_scratch[dev].norm = static_cast<double*>(p);
         g_scratch[dev].status = reinterpret_cast<unsigned*>(static_cast<char*>(p) + (prk::NORM_BLOCKS + 1) * sizeof(double));
         g_scratch[dev].context = prk::current_context_id();
@@ -135,7 +154,8 @@ int launch_one(int pattern, int radius, int64_t n, int dtype, const void* in, vo
     prk::StencilCall c{pattern, radius, n, dtype, in, in_next, out, s};
     const bool tiles = g_kernel_choice != 1 && !t_force_generic;
     const bool tma = tiles && prk::tma_eligible(c);
-    if (g_kernel_choice == 2 && !tma) return fail(PRK_ERR_ARG, "the TMA tile kernel was required but the call is not eligible");
+    // TMA required: the fused form only, as the setting has always meant
+    if (g_kernel_choice == 2 && (!tma || !in_next)) return fail(PRK_ERR_ARG, "the TMA tile kernel was required but the call is not eligible");
     if (tma) {
         DevScratch d;
         if (int rc = dev_scratch(&d)) return rc;

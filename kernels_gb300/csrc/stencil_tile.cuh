@@ -19,7 +19,7 @@
 // every tap. `out` stays in registers and is rounded after each application as the reference
 // rounds it. HBM traffic per application drops by STEPS. STEPS = 0 takes the depth at run time
 // (`depth`, any count): a whole run in one launch per tile, as the host-buffer path uses it on
-// bands of rows.
+// bands of rows. STEPS = OPERATOR is the reference operator alone: out += S(in), no in_next.
 //
 // Evaluation modes:
 //   FP64, strict   every point in the reference order with binary64 instructions (bit-exact)
@@ -58,6 +58,13 @@ struct Cfg<FP32C, TH_> {
 };
 constexpr int TH_DEFAULT = 32;
 constexpr int TH_TALL = 64;
+// STEPS of the operator form: one application of out += S(in), in untouched and no in_next. It takes
+// the same tiles and routes as the fused form and stores no in_next, so a power-of-two stencil moves 24
+// bytes per point at the copy rate: at n=8192, FP64, star R=2 2049 us on the generic kernels, 232 us
+// here (6.9 TB/s); grid R=4 18273 against 4044 us; FP32C star R=2 369 against 196 us, grid R=5 1677
+// against 599 us.
+constexpr int OPERATOR = -1;
+constexpr bool one_application(int steps) { return steps == 1 || steps == OPERATOR; }
 // Deepest run-time depth for which the FP32 route holds: 15 * (2^20 + 65536) < 2^24.
 constexpr int FP32_MAX_STEPS = 65536;
 
@@ -271,6 +278,63 @@ __device__ __forceinline__ void fp32c_points(const float* s, int ld, float (&sh)
                 two_sum(sh[k], p, t, e);
                 sh[k] = t;
                 sl[k] = __fadd_rn(sl[k], __fadd_rn(e, pe));
+            }
+        }
+    }
+}
+
+// The same sums with one compensated product per tap (fp32c_point's terms, row by row so that every
+// row segment is read once as vectors): each tap's difference enters with its own product, so no
+// difference is rounded twice.
+template <int P, int R, int CPT, int RA>
+__device__ __forceinline__ void fp32c_taps(const float* s, int ld, float (&sh)[CPT], float (&sl)[CPT])
+{
+    constexpr int SEG = CPT + 2 * RA;
+    bool first = true;  // known once the loops unroll
+    auto tap = [&](double w, const float (&d)[CPT]) {
+        const float wh = split_hi(w), wl = split_lo(w);
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) {
+            const float p = __fmul_rn(wh, d[k]);
+            float pe = __fmaf_rn(wh, d[k], -p);
+            pe = __fmaf_rn(wl, d[k], pe);
+            if (first) {
+                sh[k] = p;
+                sl[k] = pe;
+            } else {
+                float t, e;
+                two_sum(sh[k], p, t, e);
+                sh[k] = t;
+                sl[k] = __fadd_rn(sl[k], __fadd_rn(e, pe));
+            }
+        }
+        first = false;
+    };
+    {
+        float m0[SEG];
+        ld_seg<SEG>(s - RA, m0);
+#pragma unroll
+        for (int dc = 1; dc <= R; ++dc) {
+            float d[CPT];
+#pragma unroll
+            for (int k = 0; k < CPT; ++k) d[k] = __fsub_rn(m0[k + RA + dc], m0[k + RA - dc]);
+            tap(weight(P, R, dc, 0), d);
+        }
+    }
+#pragma unroll
+    for (int dr = 1; dr <= R; ++dr) {
+        constexpr int PAD = P == STAR ? 0 : RA;
+        float up[CPT + 2 * PAD], dn[CPT + 2 * PAD];
+        ld_seg<CPT + 2 * PAD>(s + dr * ld - PAD, up);
+        ld_seg<CPT + 2 * PAD>(s - dr * ld - PAD, dn);
+#pragma unroll
+        for (int dc = P == STAR ? 0 : -R; dc <= (P == STAR ? 0 : R); ++dc) {
+            const double w = weight(P, R, dc, dr);
+            if (w != 0.0) {
+                float d[CPT];
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) d[k] = __fsub_rn(up[k + PAD + dc], dn[k + PAD - dc]);
+                tap(w, d);
             }
         }
     }
@@ -1047,7 +1111,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                                              bool vec_ok, int depth, int64_t goff, int64_t row_end,
                                              unsigned char* tbl)
 {
-    const int nsteps = STEPS > 0 ? STEPS : depth;
+    const int nsteps = STEPS > 0 ? STEPS : (STEPS == OPERATOR ? 1 : depth);
     using G = Geo<DT, R, TH_>;
     using C = Cfg<DT, TH_>;
     using T = typename C::T;
@@ -1227,7 +1291,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             }
             // kernels that keep out in HBM give the route an out area right after the tables
             uint64_t* o_s = OUT_SRC == OUT_SMEM ? o_tile : reinterpret_cast<uint64_t*>(tbl + table_bytes<P, R, DT>());
-            tbl_done = table_tile<P, R, G::SW, G::SH, C::TW, ROWS, OUT_SRC, STEPS == 1>(
+            tbl_done = table_tile<P, R, G::SW, G::SH, C::TW, ROWS, OUT_SRC, one_application(STEPS)>(
                 reinterpret_cast<int32_t*>(s_in), o_s, static_cast<uint64_t*>(out_v) + i0 * n + j0, tbl, lo, hi,
                 nsteps, i0, j0, n, goff, row_end, has_out, &iw_fin);
         }
@@ -1235,6 +1299,30 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
 
     // The table route with out in HBM has stored out itself; the stores then write in_next only
     const bool out_via_rows = !(tbl_done && OUT_SRC != OUT_SMEM);
+
+    // ---- FP32C, the operator form: one compensated product per tap, or per weight group ----
+    // fp32c_points sums a weight group's differences before the product, which is exact for whole
+    // numbers near one another but rounds once per tap for others; the operator form takes the
+    // per-tap products (fp32c_taps) there. A tile takes the group sums when every value is a whole
+    // number below 2^22 within 2^18 of the tile's first: its differences stay below 2^19 and a
+    // group's sum of at most 18 of them (grid R=5, sides of ring 5) below 2^24.
+    bool grouped = true;
+    if constexpr (DT == FP32C && STEPS == OPERATOR) {
+        constexpr int NV = G::ELEMS / 4;
+        static_assert(G::ELEMS % 4 == 0, "the check reads 16-byte vectors");
+        const float ref = s_in[R * G::SW + G::RA];
+        bool ok = true;
+        for (int idx = threadIdx.x; idx < NV; idx += THREADS) {
+            const float4 v = reinterpret_cast<const float4*>(s_in)[idx];
+            const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float whole = __fsub_rn(__fadd_rn(e[k], 12582912.0f), 12582912.0f);  // |e| < 2^22
+                ok = ok && fabsf(e[k]) < 4194304.0f && whole == e[k] && fabsf(__fsub_rn(e[k], ref)) < 262144.0f;
+            }
+        }
+        grouped = __syncthreads_and(ok) != 0;
+    }
 
     // Set by the multi-application FP32 route when the tile's out words are held as integers
     bool oint = false;
@@ -1299,12 +1387,16 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         } else {
             const float* sp = reinterpret_cast<const float*>(s_in) + soff;
             float sh[CPT], sl[CPT];
-            fp32c_points<P, R, CPT, G::RA>(sp, G::SW, sh, sl);
+            if (grouped) {
+                fp32c_points<P, R, CPT, G::RA>(sp, G::SW, sh, sl);
+            } else {
+                if constexpr (STEPS == OPERATOR) fp32c_taps<P, R, CPT, G::RA>(sp, G::SW, sh, sl);
+            }
 #pragma unroll
             for (int k = 0; k < CPT; ++k) {
                 float oh = __uint_as_float(static_cast<uint32_t>(o[k]));
                 float ol = __uint_as_float(static_cast<uint32_t>(o[k] >> 32));
-                if constexpr (STEPS == 1)
+                if constexpr (one_application(STEPS))
                     df_add(oh, ol, sh[k], sl[k]);
                 else  // out stays in registers: renormalised once, before it is stored
                     df_add_lazy(oh, ol, sh[k], sl[k]);
@@ -1316,54 +1408,56 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
     // in_next (in + 1 after the last application) and out of row r to HBM
     auto store_row = [&](int r, const uint64_t* o, bool row_out) {
         const int64_t gi = i0 + r;
-        const int soff = (r + R) * G::SW + G::RA + c0;
-        T nxt[CPT];
-        bool done = false;
-        if constexpr (EXACT) {
-            if (fexact) {
-                const float* v = reinterpret_cast<const float*>(s_in) + fin_off + soff;
+        if constexpr (STEPS != OPERATOR) {
+            const int soff = (r + R) * G::SW + G::RA + c0;
+            T nxt[CPT];
+            bool done = false;
+            if constexpr (EXACT) {
+                if (fexact) {
+                    const float* v = reinterpret_cast<const float*>(s_in) + fin_off + soff;
 #pragma unroll
-                for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(f2d(__fadd_rn(v[k], 1.0f), 0));
-                done = true;
-            } else if (unit != fx::NOT_FIXED) {
-                const int64_t* v = reinterpret_cast<const int64_t*>(s_in) + soff;
-                const int64_t one = 1ll << (-unit);
-                if (narrow) {
+                    for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(f2d(__fadd_rn(v[k], 1.0f), 0));
+                    done = true;
+                } else if (unit != fx::NOT_FIXED) {
+                    const int64_t* v = reinterpret_cast<const int64_t*>(s_in) + soff;
+                    const int64_t one = 1ll << (-unit);
+                    if (narrow) {
 #pragma unroll
-                    for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(from_fixed32(static_cast<int32_t>(v[k] + one), unit));
-                } else {
+                        for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(from_fixed32(static_cast<int32_t>(v[k] + one), unit));
+                    } else {
 #pragma unroll
-                    for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(fx::from_fixed(v[k] + one, unit));
+                        for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(fx::from_fixed(v[k] + one, unit));
+                    }
+                    done = true;
                 }
-                done = true;
             }
-        }
-        if constexpr (DT == FP64 && !EXACT) {
-            if (iwhole) {
-                const int32_t* v = reinterpret_cast<const int32_t*>(s_in) + iw_fin + soff;
+            if constexpr (DT == FP64 && !EXACT) {
+                if (iwhole) {
+                    const int32_t* v = reinterpret_cast<const int32_t*>(s_in) + iw_fin + soff;
 #pragma unroll
-                for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(from_fixed32(v[k] + 1, 0));
-                done = true;
+                    for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(from_fixed32(v[k] + 1, 0));
+                    done = true;
+                }
             }
-        }
-        if (!done) {
+            if (!done) {
 #pragma unroll
-            for (int k = 0; k < CPT; ++k) {
-                if constexpr (DT == FP64)
-                    nxt[k] = inc_exact(s_in[soff + k]);
-                else
-                    nxt[k] = __fadd_rn(s_in[soff + k], 1.0f);
+                for (int k = 0; k < CPT; ++k) {
+                    if constexpr (DT == FP64)
+                        nxt[k] = inc_exact(s_in[soff + k]);
+                    else
+                        nxt[k] = __fadd_rn(s_in[soff + k], 1.0f);
+                }
             }
-        }
-        T* nx = static_cast<T*>(in_next_v) + gi * n + gj;
-        // 16-byte stores wherever the row's words start on a 16-byte boundary inside the grid (every
-        // row for the TMA tiles; every other row for an odd n)
-        if (vec_ok || (gj + CPT <= n && (reinterpret_cast<uintptr_t>(nx) & 15u) == 0)) {
-            st_vec(nx, nxt);
-        } else {
+            T* nx = static_cast<T*>(in_next_v) + gi * n + gj;
+            // 16-byte stores wherever the row's words start on a 16-byte boundary inside the grid (every
+            // row for the TMA tiles; every other row for an odd n)
+            if (vec_ok || (gj + CPT <= n && (reinterpret_cast<uintptr_t>(nx) & 15u) == 0)) {
+                st_vec(nx, nxt);
+            } else {
 #pragma unroll
-            for (int k = 0; k < CPT; ++k)
-                if (gj + k < n) nx[k] = nxt[k];
+                for (int k = 0; k < CPT; ++k)
+                    if (gj + k < n) nx[k] = nxt[k];
+            }
         }
         if (row_out) {
             uint64_t* out = static_cast<uint64_t*>(out_v) + gi * n + gj;
@@ -1378,7 +1472,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         }
     };
 
-    if constexpr (STEPS == 1) {
+    if constexpr (one_application(STEPS)) {
         // one pass: each row's new out and in_next leave as soon as they are computed. OUT_HBM_AHEAD:
         // every row's out words are requested first, so that their latencies overlap instead of
         // stalling each row in turn.
@@ -1594,11 +1688,11 @@ constexpr int min_blocks()
     // R=3..5: at three, grid R=5 spilled 3 KB)
     if (DT == FP64 && !pow2_weights(P, R)) {
         if (SMEM_PER_SM / (tile_smem<P, R, DT, TH_>() + 1024) < 3) return 2;
-        return STEPS == 1 ? PRK_STRICT_BLOCKS_1 : PRK_STRICT_BLOCKS_N;
+        return one_application(STEPS) ? PRK_STRICT_BLOCKS_1 : PRK_STRICT_BLOCKS_N;
     }
     if (DT == FP32C && P == GRID && R >= 3) return 2;  // bound by FP32 issue: registers over residency
     const int b = Geo<DT, R, TH_>::CTAS;
-    if (STEPS == 1) return b;
+    if (one_application(STEPS)) return b;
     const int cap = DT == FP64 ? 4 : 3;  // FP64 power-of-two: the FP32 route is shared-memory bound
     return b < cap ? b : cap;
 }
@@ -1681,6 +1775,11 @@ cudaError_t launch_pattern(int R, int steps, const Launch& L)
         case 0:                                                  \
             if constexpr (TH_ == TH_DEFAULT)                     \
                 return launch<P, RR, DT, 0, TH_>(L);             \
+            else                                                 \
+                return cudaErrorInvalidValue;                    \
+        case OPERATOR:                                           \
+            if constexpr (TH_ == TH_DEFAULT)                     \
+                return launch<P, RR, DT, OPERATOR, TH_>(L);      \
             else                                                 \
                 return cudaErrorInvalidValue;                    \
         default: return cudaErrorInvalidValue;                   \

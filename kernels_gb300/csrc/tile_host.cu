@@ -74,7 +74,6 @@ cudaError_t launch_wait_selftest(unsigned* status, cudaStream_t s)
 
 bool tma_eligible(const StencilCall& c)
 {
-    if (!c.in_next) return false;  // the reference-operator form (no in_next) uses the generic kernel
     const int vec = c.dtype == FP64 ? 2 : 4;
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     return c.n % vec == 0 && c.n >= 8 && al16(c.in) && al16(c.in_next) && al16(c.out);
@@ -111,12 +110,16 @@ cudaError_t launch_tma(const StencilCall& c, int steps, unsigned* status, int ti
 cudaError_t launch_stencil_tma(const StencilCall& c, int steps, unsigned* status, int tile_rows)
 {
     if (!tma_depth_ok(steps) || !tma_rows_ok(tile_rows)) return cudaErrorInvalidValue;
+    if (!c.in_next) {  // the operator form: 32-row tiles only
+        if (steps != 1) return cudaErrorInvalidValue;
+        return launch_tma(c, tile::OPERATOR, status, tile::TH_DEFAULT, 0, 0, 0);
+    }
     return launch_tma(c, steps, status, tile_rows, 0, 0, 0);
 }
 
 bool plain_eligible(const StencilCall& c)
 {
-    if (!c.in_next || c.n > NMAX) return false;
+    if (c.n > NMAX) return false;
     auto al = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
     const uintptr_t e = c.dtype == FP64 ? 8 : 4;
     return al(c.in, e) && al(c.in_next, e) && al(c.out, 8);
@@ -124,7 +127,7 @@ bool plain_eligible(const StencilCall& c)
 
 cudaError_t launch_stencil_plain(const StencilCall& c, int depth, int64_t row0, int64_t rows)
 {
-    if (depth < 1 || !plain_eligible(c)) return cudaErrorInvalidValue;
+    if (depth < 1 || (!c.in_next && depth != 1) || !plain_eligible(c)) return cudaErrorInvalidValue;
     const plain::Args a{c.in, c.in_next, c.out, c.n, depth, c.stream, row0, rows, c.nr, c.goff};
     return c.dtype == FP64 ? plain::launch_fp64(c.pattern, c.R, a) : plain::launch_fp32c(c.pattern, c.R, a);
 }

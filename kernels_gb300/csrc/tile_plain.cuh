@@ -7,7 +7,7 @@
 // that take the table route, and the tile is evaluated by the same code as the TMA and batched
 // kernels (stencil_tile.cuh): the same exact routes, the same certification.
 // STEPS = 1 is one application per launch; STEPS = 0 takes the number of applications at run time
-// (any temporal depth, or a whole run).
+// (any temporal depth, or a whole run); STEPS = tile::OPERATOR is the reference operator alone.
 #pragma once
 
 #include "batch_kernel.cuh"
@@ -37,7 +37,7 @@ template <int P, int R, int DT, int STEPS>
 constexpr int plain_min_blocks()
 {
     constexpr int b = tile::min_blocks<P, R, DT, STEPS, tile::TH_DEFAULT>();
-    return DT == FP64 && pow2_weights(P, R) && STEPS == 1 && b > 5 ? 5 : b;
+    return DT == FP64 && pow2_weights(P, R) && tile::one_application(STEPS) && b > 5 ? 5 : b;
 }
 
 // Stage the tile with asynchronous copies (cp.async), one element each: the `in` tile with its halo
@@ -165,12 +165,15 @@ cudaError_t launch(const Args& a)
     return cudaGetLastError();
 }
 
-// One application (depth 1: the STEPS = 1 kernel) or `depth` applications in one launch (STEPS = 0).
+// One application (depth 1: the STEPS = 1 kernel), `depth` applications in one launch (STEPS = 0), or
+// the operator form (no in_next).
 template <int DT>
 cudaError_t launch_form(int pattern, int R, const Args& a)
 {
 #define PRK_PLAIN(PP, RR) \
-    case RR: return a.depth == 1 ? launch<PP, RR, DT, 1>(a) : launch<PP, RR, DT, 0>(a);
+    case RR:                                                                       \
+        if (!a.in_next) return launch<PP, RR, DT, tile::OPERATOR>(a);               \
+        return a.depth == 1 ? launch<PP, RR, DT, 1>(a) : launch<PP, RR, DT, 0>(a);
     if (pattern == STAR) {
         switch (R) { PRK_PLAIN(STAR, 1) PRK_PLAIN(STAR, 2) PRK_PLAIN(STAR, 3) PRK_PLAIN(STAR, 4) PRK_PLAIN(STAR, 5) }
     } else {
