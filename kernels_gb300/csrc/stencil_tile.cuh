@@ -542,6 +542,14 @@ __device__ __forceinline__ uint64_t from_fixed32(int32_t x, int unit)
     return s | ((static_cast<uint64_t>(msb + unit + 1022) << 52) + m);
 }
 
+// binary64 encoding of a whole number |v| < 2^22, through the float it is exactly: a magic number's
+// mantissa takes the integer and one FP32 subtraction normalises it, where from_fixed32 searches for
+// the leading bit and shifts 64 bits.
+__device__ __forceinline__ uint64_t whole_bits(int32_t v)
+{
+    return f2d(__fsub_rn(__uint_as_float(0x4B400000u + static_cast<uint32_t>(v)), 12582912.0f), 0);
+}
+
 // out = V * 2^-shift for an integer V with |V| < 2^21, read from the binary64 encoding (+-0 give 0);
 // false for any other value. With M the 53-bit significand, V = M >> (k + 32) for
 // k = 1043 - shift - (biased exponent), an integer below 2^21 exactly when 0 <= k <= 20 and the
@@ -776,14 +784,15 @@ constexpr int OUT_SMEM = 0, OUT_HBM = 1, OUT_HBM_AHEAD = 2;
 //    fl(|w| * v) from a shared-memory table of every weight group and every such v, built once per
 //    tile with fx::mul_whole20 (the weight's sign enters as an add or a subtract). Every tap still
 //    reads its own in value, and indexes the table with it.
-//  - The first fixed_taps() adds of each point's chain run in 96-bit fixed point on the integer
-//    pipes (fx::fx96_acc_round: the exact sum rounded to 53 bits, nearest-even, the binary64 add's
-//    result bit for bit on these values), the rest and the add into out on the binary64 pipe.
+//  - Most adds of each point's chain run in fixed point on the integer pipes, the exact sum rounded to
+//    53 bits, nearest-even: the binary64 add's result bit for bit on these values. In 64 bits where a
+//    window's values allow it (the narrow form), else in 96 (fx::fx96_acc_round). The rest, and the add
+//    into out, run on the binary64 pipe.
 // Lane l evaluates columns l and l + 32 of its warp's rows, so a warp's table reads are consecutive
 // entries; the results go into the shared-memory out tile, which the stores then read in their own
 // layout. Applications of a multi-application launch write in + 1 to the other half of the stage
-// (the int32 tile takes half of it), and the table is rebuilt at a new base when the values outgrow
-// it.
+// (the int32 tile takes half of it), and the tables are rebuilt at a new base when the values outgrow
+// them.
 
 constexpr int TBL_L = 128;  // consecutive values one product table covers
 
@@ -836,16 +845,11 @@ static_assert(strict_taps_ok<STAR, 3>() && strict_taps_ok<STAR, 4>() && strict_t
                   strict_taps_ok<GRID, 5>(),
               "strict tap groups");
 
-// Sixteenths of each chain that run in fixed point (the rest stays on the binary64 pipe), per stencil
-// and form (ONE: one application per launch; else several, where the tile's load is shared by the
-// applications and the integer pipes take more of the chain), as measured best at n=16384 among 9 to
-// 15 sixteenths (GFLOP/s, best against the next best):
-//  - one application: star R=3, 4 11/16 (2150 against 2098 at 12/16 for R=4), R=5 12/16 (2066
-//    against 2031 at 13/16); grid R=2 11/16 (2745 against 2704 at 12/16), R=3 12/16 (2870 against
-//    2859 at 11/16), R=4 13/16 (2728 against 2721 at 14/16), R=5 15/16 (2656 against 2621 at 13/16);
-//  - several (whole runs of 20): star R=3 14/16 (2777 against 2714 at 12/16), R=4, 5 13/16 (2930
-//    against 2898 at 14/16 for R=5); grid R=2, 3 12/16 (3616 against 3557 at 13/16 for R=2), R=4
-//    14/16 (3444 against 3419 at 13/16), R=5 13/16 (3222 against 3148 at 12/16).
+// Sixteenths of each chain that run in fixed point in the 96-bit form (the rest on the binary64 pipe),
+// per stencil and form (ONE: one application per launch; else several), as measured at n=16384 when
+// every tile took this form: star R=3, 4 11/16 and R=5 12/16 at one application, 14/16 and 13/16 at
+// several; grid R=2 11/16, R=3 12/16, R=4 13/16, R=5 15/16 at one, 12/16, 12/16, 14/16 and 13/16 at
+// several.
 template <int P, int R, bool ONE>
 __host__ __device__ constexpr int fixed_sixteenths()
 {
@@ -865,28 +869,26 @@ __host__ __device__ constexpr int fixed_taps()
     return k < 1 ? 1 : (k > tap_count(P, R) ? tap_count(P, R) : k);
 }
 
-// True when a positive weight lies among the fixed taps: then the fixed part never sums to -0 (a
-// rounded sum is -0 only when every term is -0, and w * v with w > 0 is never -0).
-template <int P, int R, bool ONE>
-constexpr bool fixed_prefix_has_positive()
-{
-    constexpr StrictTaps<P, R> t = make_strict_taps<P, R>();
-    for (int k = 0; k < fixed_taps<P, R, ONE>(); ++k)
-        if (!t.neg[k]) return true;
-    return false;
-}
-
 template <int P, int R, int DT>
 __host__ __device__ constexpr bool table_route()
 {
     return DT == FP64 && !pow2_weights(P, R);
 }
 
-// Shared memory of the tables: per weight group TBL_L binary64 products and TBL_L fixed-point images.
+// Shared memory of the tables: per weight group TBL_L binary64 products, then TBL_L 96-bit images or
+// TBL_L 64-bit images of either sign (the narrow form), then one descriptor per tap (the narrow form).
 template <int P, int R, int DT>
 __host__ __device__ constexpr int table_bytes()
 {
-    return table_route<P, R, DT>() ? group_count<P, R>() * TBL_L * (8 + 16) : 0;
+    return table_route<P, R, DT>() ? group_count<P, R>() * TBL_L * (8 + 16) + tap_count(P, R) * 16 : 0;
+}
+
+// Tiles of the table route resident per SM: four where their shared memory allows it (star R=3, 4, grid
+// R=2; 64 registers), else three (80).
+template <int P, int R>
+__host__ __device__ constexpr int strict_tiles()
+{
+    return 4 * (table_offset<FP64, R, 32>() + table_bytes<P, R, FP64>() + 1024) <= SMEM_PER_SM ? 4 : 3;
 }
 
 // Dynamic shared memory of the TMA kernel: its tile stages, and the tables where the route applies.
@@ -916,15 +918,6 @@ __device__ __forceinline__ void build_tables(uint64_t* T64, uint4* T96, int base
     }
 }
 
-// x = fl(x + s * p) in fixed point, s the tap's sign.
-__device__ __forceinline__ void fx96_tap(uint32_t (&x)[3], const uint4& p, int neg)
-{
-    if (neg)
-        fx::fx96_acc_round<true>(x[0], x[1], x[2], p.x, p.y, p.z);
-    else
-        fx::fx96_acc_round<false>(x[0], x[1], x[2], p.x, p.y, p.z);
-}
-
 // Where a row of the table route's points lies: a row whose points are all outside the interior or
 // past row_end is skipped (row-uniform); a column outside the interior is computed and dropped.
 __device__ __forceinline__ bool table_row_active(bool has_out, int64_t gi, int64_t gg, int64_t row_end, int64_t n, int R)
@@ -932,49 +925,300 @@ __device__ __forceinline__ bool table_row_active(bool has_out, int64_t gi, int64
     return has_out && gi < row_end && gg >= R && gg < n - R;
 }
 
-// The chain S of the points (r, c) and (r, c + 32): the reference's sum of fl(w * v) over the taps in
-// the generator's order, the adds of its first fixed_taps<P, R, ONE>() taps in fixed point. sp points
-// at the int32 tile's (r, c) (row stride SW); the tables cover [base, base + TBL_L).
-template <int P, int R, int SW, bool ONE>
-__device__ __forceinline__ void table_chain(const int32_t* sp, const uint64_t* T64, const uint4* T96, int base,
-                                            double (&d)[2])
+// The narrow form of the table route: the chain in 64-bit fixed point, its rounding positions known
+// per tap before the points are evaluated.
+//
+// In a window [base, top] of values, all of one sign, every product is a multiple of 2^L, L the lowest
+// bit of the smallest one, and so is every rounded partial sum. The partial sum after tap t lies within
+// W_t * mid +- A_t * half of the window's middle and half width (W_t, A_t the prefix sums of the weights
+// and of their magnitudes), so
+//  - where that stays below 2^62 units the sums are 64-bit integers, two words instead of three;
+//  - where it stays inside one binade, as it does unless the window straddles a power of two, the
+//    rounding position is the same for every point and comes from the tap's descriptor: no search for
+//    the leading bit, no per-point masks. The other taps find it per point (bfind).
+// Over the tiles of a PRK field at n=16384, 96% of the taps of star R=3 and 93% of grid R=5's have one
+// rounding position; at n=4096 88% and 78%. Windows that hold zero, or span too many binades, take the
+// 96-bit form (table_chain).
+//
+// A tap is a loop iteration over eight points of a thread, which share its constants and descriptor, so
+// the code stays small at 110 taps; the tile holds table offsets instead of values, so a point's two
+// reads need no address arithmetic between them. What bounds it (ncu, grid R=5, n=8192, four
+// applications): shared memory 91% of its wavefronts (one for the offset, two for the product, per 32
+// points and tap) and the integer ALU 77%, 11.6 instructions per point and tap. At n=8192, us per
+// application, against the 96-bit form for every tile: one per launch, star R=3 920 to 646, grid R=2
+// 1289 to 842, grid R=5 6448 to 3128; whole runs of 16, star R=3 604 to 429, grid R=5 4594 to 2901.
+// Slower: two products prefetched a tap ahead (grid R=2 888 and 722 at 24 warps), indices of four rows
+// packed in a word (grid R=5 3106: fewer wavefronts, more ALU instructions), the tie found through a
+// carry of the lowest kept bit (7 instructions, 3088).
+
+// Taps of each chain whose adds run in fixed point; the ones after them, at least one, run on the
+// binary64 pipe beside the integer pipes. Measured at n=8192 (us per application): one application per
+// launch, star one tap (R=3: 646 against 681 with two), grid R=2 two (842; 848 with one, 870 with
+// three), grid R=3..5 three for each ring past the second (R=5: 3128 with nine, 3154 with twelve, 3180
+// with six); several applications per launch, one (grid R=5 whole run 2901; 2939 with five).
+template <int P, int R, bool ONE>
+__host__ __device__ constexpr int narrow_taps()
 {
-    constexpr StrictTaps<P, R> TP = make_strict_taps<P, R>();
-    constexpr int N = tap_count(P, R), KF = fixed_taps<P, R, ONE>();
-    constexpr bool POS = fixed_prefix_has_positive<P, R, ONE>();
-    uint32_t x[2][3];
-    int anyv[2] = {0, 0};
+    return tap_count(P, R) - (!ONE || P == STAR ? 1 : R == 2 ? 2 : 3 * (R - 2));
+}
+
+struct alignas(16) NarrowTap {
+    int off;        // offset in the int32 tile
+    uint32_t t64;   // byte offset of the tap's binary64 products in the tables
+    uint32_t fix;   // byte offset of its signed 64-bit images
+    uint32_t sign;  // 0x80000000 for a negative weight
+};
+
+template <int P, int R, int SW>
+struct NarrowTaps {
+    NarrowTap tap[tap_count(P, R)];
+    float w[tap_count(P, R)], a[tap_count(P, R)];  // W_t and A_t
+    double gw[group_count<P, R>()];                // |weight| of each group
+};
+
+template <int P, int R, int SW>
+constexpr NarrowTaps<P, R, SW> make_narrow_taps()
+{
+    constexpr StrictTaps<P, R> s = make_strict_taps<P, R>();
+    constexpr int NG = group_count<P, R>();
+    NarrowTaps<P, R, SW> t{};
+    double w = 0.0, a = 0.0;
+    for (int k = 0; k < tap_count(P, R); ++k) {
+        t.tap[k].off = s.dr[k] * SW + s.dc[k];
+        t.tap[k].t64 = static_cast<uint32_t>(s.g[k] * TBL_L * 8);
+        t.tap[k].fix = static_cast<uint32_t>((NG + (s.neg[k] ? NG : 0) + s.g[k]) * TBL_L * 8);
+        t.tap[k].sign = s.neg[k] ? 0x80000000u : 0u;
+        const double wk = weight(P, R, s.dc[k], s.dr[k]);
+        w += wk;
+        a += wk < 0.0 ? -wk : wk;
+        t.w[k] = static_cast<float>(w);
+        t.a[k] = static_cast<float>(a);
+    }
+    for (int g = 0; g < NG; ++g) t.gw[g] = group_weight<P, R>(g);
+    return t;
+}
+
+template <int P, int R, int SW>
+__constant__ NarrowTaps<P, R, SW> c_narrow = make_narrow_taps<P, R, SW>();
+
+// Smallest weight group: its products have the lowest bits.
+template <int P, int R>
+__host__ __device__ constexpr double smallest_weight()
+{
+    double m = group_weight<P, R>(0);
+    for (int g = 1; g < group_count<P, R>(); ++g)
+        if (group_weight<P, R>(g) < m) m = group_weight<P, R>(g);
+    return m;
+}
+
+// floor(log2 x) of a positive normal float.
+__device__ __forceinline__ int log2_floor(float x) { return static_cast<int>(__float_as_uint(x) >> 23) - 127; }
+
+// Build the narrow form's tables and descriptors for the window [base, top] (top - base < TBL_L).
+// Returns false (block-uniform, through a barrier) when the window holds zero or both signs or a
+// partial sum may reach 2^62 units; *unit is L otherwise. The tables are complete on return.
+template <int P, int R, int SW, bool ONE>
+__device__ __forceinline__ bool build_narrow(unsigned char* tbl, int base, int top, int* unit)
+{
+    constexpr int NG = group_count<P, R>(), KF = narrow_taps<P, R, ONE>();
+    const int amin = base > 0 ? base : -top, amax = base > 0 ? top : -base;
+    if (amin <= 0 || amax >= (1 << 20)) return false;
+    const int L = static_cast<int>(fx::mul_whole20(encode(smallest_weight<P, R>()), amin) >> 52) - 1075;
+    uint64_t* T64 = reinterpret_cast<uint64_t*>(tbl);
+    const auto& T = c_narrow<P, R, SW>;
+#pragma unroll 1
+    for (int k = threadIdx.x; k < NG * TBL_L; k += THREADS) {
+        const int v = base + k % TBL_L;
+        const uint64_t p =
+            v <= top ? as_bits(__dmul_rn(T.gw[k / TBL_L], as_dbl(whole_bits(v)))) : 0ull;  // v is not 0
+        // p = m * 2^(e - 1075); as an integer of 2^L units m << (e - 1075 - L). The shift lies in 0..11
+        // for every product of a window that passes the check below.
+        const uint64_t m = (p & fx::MANT) | fx::HIDDEN;
+        const int sh = min(static_cast<int>((p >> 52) & 0x7FFu) - 1075 - L, 11);
+        int64_t x = p == 0 ? 0 : static_cast<int64_t>(m << (sh & 63));
+        if (p & fx::SIGN) x = -x;
+        T64[k] = p;
+        T64[NG * TBL_L + k] = static_cast<uint64_t>(x);
+        T64[2 * NG * TBL_L + k] = static_cast<uint64_t>(-x);
+    }
+    bool ok = true;
+    uint4* desc = reinterpret_cast<uint4*>(tbl + NG * TBL_L * 24);
+    for (int t = threadIdx.x; t < KF; t += THREADS) {
+        // every partial sum lies in [|W mid| - r, |W mid| + r]; the slack covers the float arithmetic
+        // and the roundings of the sum itself
+        const float mid = 0.5f * static_cast<float>(base + top), half = 0.5f * static_cast<float>(top - base);
+        const float c = fabsf(T.w[t] * mid), r = T.a[t] * (half + 1e-5f * static_cast<float>(amax));
+        const int bhi = max(log2_floor(c + r) - 52 - L, 0);
+        const int blo = c - r > 1e-3f ? max(log2_floor(c - r) - 52 - L, 0) : 0;
+        ok = ok && log2_floor(c + r) - L < 62;
+        const int b = bhi & 31;
+        desc[t] = make_uint4((1u << b) >> 1, b ? 1u << b : 0u, b ? ~((2u << b) - 1u) : ~0u, bhi != blo ? 1u : 0u);
+    }
+    *unit = L;
+    return __syncthreads_and(ok) != 0;
+}
+
+// binary64 encoding of x * 2^unit for a 64-bit x with at most 53 significant bits (0 gives +0).
+__device__ __forceinline__ uint64_t fx64_to_bits(uint32_t x0, uint32_t x1, int unit)
+{
+    const int64_t x = static_cast<int64_t>((static_cast<uint64_t>(x1) << 32) | x0);
+    if (x == 0) return 0;
+    const uint64_t a = x < 0 ? static_cast<uint64_t>(-x) : static_cast<uint64_t>(x);
+    const int lead = fx::clz64(a);
+    return (static_cast<uint64_t>(x1 >> 31) << 63) |
+           ((static_cast<uint64_t>(63 - lead + unit + 1022) << 52) + ((a << lead) >> 11));
+}
+
+// The int32 tile as byte offsets into a table of the window: 8 (v - base), and back. In place, as
+// 16-byte vectors; each thread its own.
+template <int ELEMS, bool TO>
+__device__ __forceinline__ void offsets_tile(int32_t* p, int base)
+{
+    constexpr int NV = ELEMS / 4;
+    auto f = [&](int v) { return TO ? (v - base) * 8 : (v >> 3) + base; };
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < NV; idx += THREADS) {
+        int4 v = reinterpret_cast<int4*>(p)[idx];
+        v.x = f(v.x);
+        v.y = f(v.y);
+        v.z = f(v.z);
+        v.w = f(v.w);
+        reinterpret_cast<int4*>(p)[idx] = v;
+    }
+}
+
+// The chains of a thread's eight points: rows r, r + QR, r + 2 QR, r + 3 QR (q >> 1) of columns c and
+// c + 32 (q & 1); sp points at (r, c) of the tile of table offsets. The add of tap t rounds the 64-bit sum to a
+// multiple of 2^b, nearest-even, b from the descriptor (.x = 2^(b-1), .y = 2^b, .z = the bits above b; 0,
+// 0 and all ones for b = 0): plus half a unit, then the bits below b cut (halves round up), and bit b
+// cleared on a tie. A tie leaves zeros below b, so subtracting 1 turns bit b over exactly then: bit b of
+// s & (s - 1) is the even neighbour's, and no carry leaves the low word (b <= 9).
+template <int P, int R, int SW, int QR, bool ONE>
+__device__ __forceinline__ void narrow_chain(const int32_t* sp, const unsigned char* tbl, int unit, double (&d)[8])
+{
+    constexpr int N = tap_count(P, R), KF = narrow_taps<P, R, ONE>(), NG = group_count<P, R>(), NQ = 8;
+    static_assert(N >= KF + 1 && KF >= 2, "at least one tap on the binary64 pipe");
+    const auto& T = c_narrow<P, R, SW>;
+    const uint4* desc = reinterpret_cast<const uint4*>(tbl + NG * TBL_L * 24);
+    auto load_v = [&](int t, uint32_t (&v)[NQ]) {
+        const int32_t* s = sp + T.tap[t].off;
 #pragma unroll
-    for (int t = 0; t < KF; ++t) {
+        for (int q = 0; q < NQ; ++q) v[q] = static_cast<uint32_t>(s[(q >> 1) * QR * SW + 32 * (q & 1)]);
+    };
+    auto load_p = [&](uint32_t table, const uint32_t (&v)[NQ], uint2 (&p)[NQ]) {
+        const unsigned char* tf = tbl + table;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int v = sp[TP.dr[t] * SW + TP.dc[t] + 32 * h];
-            if (!POS) anyv[h] |= v;
-            const uint4 p = T96[TP.g[t] * TBL_L + (v - base)];
-            if (t == 0) {
-                if (TP.neg[t]) {  // x = -p, the 96-bit two's-complement negation
-                    x[h][0] = ~p.x + 1u;
-                    x[h][1] = ~p.y + (p.x == 0u ? 1u : 0u);
-                    x[h][2] = ~p.z + ((p.x | p.y) == 0u ? 1u : 0u);
-                } else {
-                    x[h][0] = p.x;
-                    x[h][1] = p.y;
-                    x[h][2] = p.z;
-                }
-            } else {
-                fx96_tap(x[h], p, TP.neg[t]);
+        for (int q = 0; q < NQ; ++q) p[q] = *reinterpret_cast<const uint2*>(tf + v[q]);
+    };
+    uint32_t x0[NQ], x1[NQ], v[NQ];
+    uint2 p[NQ];
+    load_v(0, v);
+    load_p(T.tap[0].fix, v, p);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        x0[q] = p[q].x;
+        x1[q] = p[q].y;
+    }
+    load_v(1, v);  // one tap ahead
+    // two taps per trip where three tiles per SM leave the registers for it (n=8192, whole run of 16,
+    // grid R=5: 2939 us per application against 2972)
+    constexpr int UNR = strict_tiles<P, R>() == 4 ? 1 : 2;
+#pragma unroll UNR
+    for (int t = 1; t < KF; ++t) {
+        const uint4 ds = desc[t];
+        load_p(T.tap[t].fix, v, p);
+        load_v(t + 1, v);
+        if (ds.w == 0u) {  // one rounding position for the whole window
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const uint64_t s = ((static_cast<uint64_t>(x1[q]) << 32) | x0[q]) +
+                                   ((static_cast<uint64_t>(p[q].y) << 32) | p[q].x) + ds.x;
+                x1[q] = static_cast<uint32_t>(s >> 32);
+                x0[q] = static_cast<uint32_t>(s);
+                x0[q] &= ((x0[q] - 1u) & ds.y) | ds.z;
+            }
+        } else {  // from each sum's leading bit (bits 52 and up of |sum| lie in the high word)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                uint64_t s = ((static_cast<uint64_t>(x1[q]) << 32) | x0[q]) +
+                             ((static_cast<uint64_t>(p[q].y) << 32) | p[q].x);
+                int f;
+                asm("bfind.s32 %0, %1;" : "=r"(f) : "r"(static_cast<uint32_t>(s >> 32)));
+                const uint32_t bit = 1u << max(f - 20, 0);  // 2^b
+                const uint32_t c = bit - 1u, c2 = c << 1;
+                s += bit >> 1;
+                x1[q] = static_cast<uint32_t>(s >> 32);
+                x0[q] = static_cast<uint32_t>(s);
+                x0[q] &= ((x0[q] - 1u) & (c2 & ~c)) | ~(c | c2);
             }
         }
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) d[h] = as_dbl(fx::fx96_to_bits(x[h][0], x[h][1], x[h][2], !POS && anyv[h] == 0));
-#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if constexpr (ONE) {
+            // One conversion instruction (it runs on the binary64 pipe, which has room at one application
+            // per launch), exact for 53 significant bits, then the unit into the exponent.
+            const uint64_t b = as_bits(__ll2double_rn(static_cast<long long>((static_cast<uint64_t>(x1[q]) << 32) | x0[q])));
+            d[q] = as_dbl(b == 0 ? 0ull : b + (static_cast<uint64_t>(static_cast<int64_t>(unit)) << 52));
+        } else {
+            d[q] = as_dbl(fx64_to_bits(x0[q], x1[q], unit));
+        }
+    }
+#pragma unroll 1
     for (int t = KF; t < N; ++t) {
+        const NarrowTap tp = T.tap[t];
+        load_v(t, v);
+        load_p(tp.t64, v, p);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int v = sp[TP.dr[t] * SW + TP.dc[t] + 32 * h];
-            const double p = as_dbl(T64[TP.g[t] * TBL_L + (v - base)]);
-            d[h] = TP.neg[t] ? __dsub_rn(d[h], p) : __dadd_rn(d[h], p);
+        for (int q = 0; q < NQ; ++q)
+            d[q] = __dadd_rn(d[q], as_dbl((static_cast<uint64_t>(p[q].y ^ tp.sign) << 32) | p[q].x));
+    }
+}
+
+// The chains of four points in 96-bit fixed point: rows r and r + WARPS (q >> 1) of columns c and c + 32
+// (q & 1); sp points at (r, c) of the int32 tile, the tables cover [base, base + TBL_L). The adds of the
+// first fixed_taps<P, R, ONE>() taps run in fixed point (fx::fx96_acc_round), the rest on the binary64
+// pipe. A tap is a loop iteration, as in the narrow form: windows that take this form are few (those
+// that hold zero), and unrolled taps cost every kernel of the stencil registers and code. A rounded sum
+// is -0 only when every term is -0: no positive weight and no value but zero so far.
+template <int P, int R, int SW, bool ONE>
+__device__ __forceinline__ void table_chain(const int32_t* sp, const unsigned char* tbl, int base, double (&d)[4])
+{
+    constexpr int N = tap_count(P, R), KF = fixed_taps<P, R, ONE>(), NG = group_count<P, R>(), NQ = 4;
+    const auto& T = c_narrow<P, R, SW>;
+    uint32_t x[NQ][3] = {};
+    int anyv[NQ] = {};
+    bool positive = false;
+    auto value = [&](const int32_t* s, int q) { return s[(q >> 1) * WARPS * SW + 32 * (q & 1)]; };
+#pragma unroll 1
+    for (int t = 0; t < KF; ++t) {
+        const NarrowTap tp = T.tap[t];
+        const int32_t* s = sp + tp.off;
+        const unsigned char* tf = tbl + NG * TBL_L * 8 + 2 * tp.t64;
+        positive = positive || tp.sign == 0u;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int v = value(s, q);
+            anyv[q] |= v;
+            const uint4 p = *reinterpret_cast<const uint4*>(tf + (v - base) * 16);
+            if (tp.sign)
+                fx::fx96_acc_round<true>(x[q][0], x[q][1], x[q][2], p.x, p.y, p.z);
+            else
+                fx::fx96_acc_round<false>(x[q][0], x[q][1], x[q][2], p.x, p.y, p.z);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+        d[q] = as_dbl(fx::fx96_to_bits(x[q][0], x[q][1], x[q][2], !positive && anyv[q] == 0));
+#pragma unroll 1
+    for (int t = KF; t < N; ++t) {
+        const NarrowTap tp = T.tap[t];
+        const int32_t* s = sp + tp.off;
+        const unsigned char* tf = tbl + tp.t64;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const uint2 p = *reinterpret_cast<const uint2*>(tf + (value(s, q) - base) * 8);
+            d[q] = __dadd_rn(d[q], as_dbl((static_cast<uint64_t>(p.y ^ tp.sign) << 32) | p.x));
         }
     }
 }
@@ -983,9 +1227,9 @@ __device__ __forceinline__ void table_chain(const int32_t* sp, const uint64_t* T
 // out in HBM (one FP64 tile of out words; the TMA kernel updates its out tile instead).
 __host__ __device__ constexpr int table_out_bytes() { return Cfg<FP64>::TW * Cfg<FP64>::TH * 8; }
 
-// dst = src + 1 over a whole int32 tile, halo included, as 16-byte vectors.
+// dst = src + one over a whole int32 tile, halo included, as 16-byte vectors.
 template <int ELEMS>
-__device__ __forceinline__ void advance_i32_to(const int32_t* src, int32_t* dst)
+__device__ __forceinline__ void advance_i32_to(const int32_t* src, int32_t* dst, int one)
 {
     constexpr int NV = ELEMS / 4;
 #pragma unroll
@@ -993,20 +1237,26 @@ __device__ __forceinline__ void advance_i32_to(const int32_t* src, int32_t* dst)
         const int idx = threadIdx.x + q * THREADS;
         if (NV % THREADS == 0 || idx < NV) {
             int4 v = reinterpret_cast<const int4*>(src)[idx];
-            v.x += 1;
-            v.y += 1;
-            v.z += 1;
-            v.w += 1;
+            v.x += one;
+            v.y += one;
+            v.z += one;
+            v.w += one;
             reinterpret_cast<int4*>(dst)[idx] = v;
         }
     }
 }
 
+// Where a whole-number tile's int32 words lie (elements from the stage) and how they hold the values:
+// value = (word >> shift) + add.
+struct WholeTile {
+    int off = 0, shift = 0, add = 0;
+};
+
 // The table route for a whole tile whose int32 values (the tile's in, halo included) lie in
 // [lo, hi]: `nsteps` applications. The int32 tile takes half of the FP64 stage, so the other half
 // holds the next application's in: while application t reads one, in + 1 goes to the other, and
-// one barrier per application separates them; *fin (0 or SW * SH) is where the last application's
-// in is left for the stores. Lane l owns columns l and l + 32 of its warp's rows; every application
+// one barrier per application separates them; *fin says where and how the last application's in is
+// left for the stores. Lane l owns columns l and l + 32 of its warp's rows; every application
 // adds its S into their out words in o_s, a shared-memory tile of out words (row stride TW). With
 // OUT_SMEM, o_s is the TMA kernel's out tile, which the stores then read in their own layout; with
 // the other sources o_s is scratch, filled from the out array (out_g points at the tile's (0, 0),
@@ -1016,7 +1266,7 @@ __device__ __forceinline__ void advance_i32_to(const int32_t* src, int32_t* dst)
 template <int P, int R, int SW, int SH, int TW, int ROWS, int OUT_SRC, bool ONE>
 __device__ __forceinline__ bool table_tile(int32_t* si, uint64_t* o_s, uint64_t* out_g, unsigned char* tbl, int lo,
                                            int hi, int nsteps, int64_t i0, int64_t j0, int64_t n, int64_t goff,
-                                           int64_t row_end, bool has_out, int* fin)
+                                           int64_t row_end, bool has_out, WholeTile* fin)
 {
     constexpr int ELEMS = SW * SH;
     static_assert(TW == 64, "two columns per lane, 32 apart");
@@ -1025,12 +1275,32 @@ __device__ __forceinline__ bool table_tile(int32_t* si, uint64_t* o_s, uint64_t*
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint64_t* T64 = reinterpret_cast<uint64_t*>(tbl);
     uint4* T96 = reinterpret_cast<uint4*>(tbl + group_count<P, R>() * TBL_L * 8);
-    int base = lo;
-    build_tables<P, R>(T64, T96, base);
+    // Application t's in is the int32 tile at si + cur: values, or (narrow) byte offsets into the
+    // window's tables. The other half of the stage takes in + 1 for application t + 1.
+    constexpr int QR = ROWS * WARPS / 4;
+    static_assert(QR % WARPS == 0, "a thread's rows in groups of four, QR apart");
+    int cur = 0, base = lo, unit = 0;
+    bool narrow = false;
+    // The tables of the window of values from application t's smallest on, complete on return: the
+    // narrow form's (with the tile turned into table offsets) where it holds, else the 96-bit form's. si is
+    // at application t.
+    auto build = [&](int t) {
+        base = lo + t;
+        narrow = build_narrow<P, R, SW, ONE>(tbl, base, min(hi + nsteps - 1, base + TBL_L - 1), &unit);
+        if (narrow) {
+            offsets_tile<ELEMS, true>(si + cur, base);
+            __syncthreads();
+        }
+        if (!narrow) {
+            __syncthreads();  // a form that was tried and given up is overwritten
+            build_tables<P, R>(T64, T96, base);
+            __syncthreads();
+        }
+    };
     if constexpr (OUT_SRC != OUT_SMEM) {
 #pragma unroll
         for (int rr = 0; rr < ROWS; ++rr) {
-            const int r = warp * ROWS + rr;
+            const int r = warp + WARPS * rr;
             const int64_t gi = i0 + r;
             if (!table_row_active(has_out, gi, gi + goff, row_end, n, R)) continue;
 #pragma unroll
@@ -1040,41 +1310,67 @@ __device__ __forceinline__ bool table_tile(int32_t* si, uint64_t* o_s, uint64_t*
             }
         }
     }
-    __syncthreads();  // the tables complete
-    int cur = 0;
+    // which of a word row's eight points are updated: bit q of the group's mask (narrow form)
+    auto active = [&](int wr) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int64_t gi = i0 + wr + (q >> 1) * QR, c = j0 + lane + 32 * (q & 1);
+            if (table_row_active(has_out, gi, gi + goff, row_end, n, R) && c >= R && c < n - R) m |= 1u << q;
+        }
+        return m;
+    };
+    const uint32_t act0 = active(warp);
+    build(0);
 #pragma unroll 1
     for (int t = 0; t < nsteps; ++t) {
         if (t > 0 && hi + t >= base + TBL_L) {  // the values outgrew the table: rebuild it at the new minimum
-            base = lo + t;
-            build_tables<P, R>(T64, T96, base);
-            __syncthreads();
+            if (narrow) offsets_tile<ELEMS, false>(si + cur, base);
+            build(t);
         }
-        const int32_t* s0 = si + cur + R * SW + ((SW - TW) / 2);  // the tile's (0, 0)
+        if (narrow) {
 #pragma unroll 1
-        for (int rr = 0; rr < ROWS; ++rr) {
-            const int r = warp * ROWS + rr;
-            const int64_t gi = i0 + r;
-            if (!table_row_active(has_out, gi, gi + goff, row_end, n, R)) continue;  // warp-uniform
-            double d[2];
-            table_chain<P, R, SW, ONE>(s0 + r * SW + lane, T64, T96, base, d);
+            for (int wr = warp; wr < QR; wr += WARPS) {
+                const uint32_t act = ROWS == 4 ? act0 : active(wr);
+                if (__ballot_sync(0xffffffffu, act != 0) == 0) continue;  // no interior point in the warp's rows
+                double d[8];
+                narrow_chain<P, R, SW, QR, ONE>(si + cur + (wr + R) * SW + (SW - TW) / 2 + lane, tbl, unit, d);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int c = lane + 32 * h;
-                if (j0 + c >= R && j0 + c < n - R)
-                    o_s[r * TW + c] = as_bits(__dadd_rn(as_dbl(o_s[r * TW + c]), d[h]));
+                for (int q = 0; q < 8; ++q) {
+                    uint64_t* o = o_s + (wr + (q >> 1) * QR) * TW + lane + 32 * (q & 1);
+                    if (act >> q & 1u) *o = as_bits(__dadd_rn(as_dbl(*o), d[q]));
+                }
+            }
+        } else {
+            const int32_t* s0 = si + cur + R * SW + ((SW - TW) / 2);  // the tile's (0, 0)
+#pragma unroll 1
+            for (int rr = 0; rr < ROWS; rr += 2) {
+                const int r = warp + WARPS * rr;
+                double d[4];
+                table_chain<P, R, SW, ONE>(s0 + r * SW + lane, tbl, base, d);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int rq = r + (q >> 1) * WARPS, c = lane + 32 * (q & 1);
+                    if (table_row_active(has_out, i0 + rq, i0 + rq + goff, row_end, n, R) && j0 + c >= R && j0 + c < n - R)
+                        o_s[rq * TW + c] = as_bits(__dadd_rn(as_dbl(o_s[rq * TW + c]), d[q]));
+                }
             }
         }
-        if (t + 1 < nsteps) {
-            advance_i32_to<ELEMS>(si + cur, si + (ELEMS - cur));
+        if (t + 1 < nsteps) {  // in += 1
+            advance_i32_to<ELEMS>(si + cur, si + (ELEMS - cur), narrow ? 8 : 1);
             cur = ELEMS - cur;
             __syncthreads();  // the next application's in complete, this one's reads done
         }
     }
-    *fin = cur;
+    // The last application's in, for the stores: value = (word >> shift) + add. The words stay as they
+    // are, as other warps may still be reading them.
+    fin->off = cur;
+    fin->shift = narrow ? 3 : 0;
+    fin->add = narrow ? base : 0;
     if constexpr (OUT_SRC != OUT_SMEM) {
 #pragma unroll
         for (int rr = 0; rr < ROWS; ++rr) {
-            const int r = warp * ROWS + rr;
+            const int r = warp + WARPS * rr;
             const int64_t gi = i0 + r;
             if (!table_row_active(has_out, gi, gi + goff, row_end, n, R)) continue;
 #pragma unroll
@@ -1235,17 +1531,31 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         const uint64_t* raw = reinterpret_cast<const uint64_t*>(s_in);
         int32_t iv[PER];
         bool ok = nsteps <= (1 << 19);
+        // Elements no stored point reads (outside the grid, or past the last row's halo) hold zeros; they
+        // stay out of the tile's range and take its lowest value, so that a tile at the grid's edge has
+        // the range of its own values. (Its halo's zeros made the range too wide for the tables: at
+        // n=1000 18% of the tiles took the product route for it.)
+        const int64_t row_hi = min(row_end + R, n - goff);  // first array row past those that are read
+        const bool edge = i0 < R || j0 < G::RA || i0 + C::TH + R > row_hi || j0 + C::TW + G::RA > n;
+        auto inside = [&](int idx) {
+            const int r = idx / G::SW, c = idx - r * G::SW;
+            return static_cast<uint64_t>(i0 - R + r) < static_cast<uint64_t>(row_hi) &&
+                   static_cast<uint64_t>(j0 - G::RA + c) < static_cast<uint64_t>(n);
+        };
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
             const int idx = threadIdx.x + q * THREADS;
             const uint64_t b = idx < G::ELEMS ? raw[idx] : 0ull;
-            const int e = static_cast<int>((b >> 52) & 0x7FF);
-            const int sh = 1075 - e;  // fraction bits below the binary point, 34..52 in range
-            const bool in_range = e >= 1023 && e <= 1041;
-            const uint64_t m = (b & fx::MANT) | fx::HIDDEN;
-            const bool whole = in_range && (m & ((1ull << (sh & 63)) - 1)) == 0;
-            const int32_t a = in_range ? static_cast<int32_t>(m >> (sh & 63)) : 0;
-            iv[q] = b == 0ull ? 0 : ((b >> 63) ? -a : a);
+            // |v| in [1, 2^19) by its exponent; then v as a float (the exponent rebiased, the fraction
+            // bits a float cannot hold checked for zero) and as an integer, rounded by the magic number
+            // and compared back
+            const uint32_t hi32 = static_cast<uint32_t>(b >> 32), lo32 = static_cast<uint32_t>(b);
+            const bool in_range = (hi32 & 0x7FFFFFFFu) - 0x3FF00000u < (19u << 20);
+            const uint32_t fb = __funnelshift_l(lo32, hi32, 3) - (128u << 23);
+            const float f = __uint_as_float((hi32 & 0x80000000u) | (fb & 0x7FFFFFFFu));
+            const float t = __fadd_rn(f, 12582912.0f);  // 1.5 * 2^23
+            const bool whole = in_range && (lo32 & 0x1FFFFFFFu) == 0u && __fsub_rn(t, 12582912.0f) == f;
+            iv[q] = whole ? static_cast<int32_t>(__float_as_uint(t) - 0x4B400000u) : 0;
             ok = ok && (b == 0ull || whole);
         }
         if constexpr (table_route<P, R, DT>()) {
@@ -1253,7 +1563,8 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             int lo = 0x7FFFFFFF, hi = -0x7FFFFFFF;
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
-                if (threadIdx.x + q * THREADS < G::ELEMS) {
+                const int idx = threadIdx.x + q * THREADS;
+                if (idx < G::ELEMS && (!edge || inside(idx))) {
                     lo = min(lo, iv[q]);
                     hi = max(hi, iv[q]);
                 }
@@ -1268,10 +1579,16 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         iwhole = __syncthreads_and(ok) != 0;
         if (iwhole) {
             int32_t* si = reinterpret_cast<int32_t*>(s_in);
+            int fill = 0;
+            if (edge) {
+                fill = s_red[0];
+#pragma unroll
+                for (int w = 1; w < WARPS; ++w) fill = min(fill, s_red[2 * w]);
+            }
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 const int idx = threadIdx.x + q * THREADS;
-                if (idx < G::ELEMS) si[idx] = iv[q];
+                if (idx < G::ELEMS) si[idx] = !edge || inside(idx) ? iv[q] : fill;
             }
         }
         __syncthreads();
@@ -1280,7 +1597,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
     // ---- FP64, other weights: the table route (table_tile), when the kernel has a table area and
     // the tile's range fits it ----
     bool tbl_done = false;
-    int iw_fin = 0;  // where the int32 tile of the last application's in lies (int32 elements)
+    WholeTile iw_fin;  // the int32 tile of the last application's in
     if constexpr (table_route<P, R, DT>()) {
         if (iwhole && tbl) {
             int lo = s_red[0], hi = s_red[1];
@@ -1433,9 +1750,9 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             }
             if constexpr (DT == FP64 && !EXACT) {
                 if (iwhole) {
-                    const int32_t* v = reinterpret_cast<const int32_t*>(s_in) + iw_fin + soff;
+                    const int32_t* v = reinterpret_cast<const int32_t*>(s_in) + iw_fin.off + soff;
 #pragma unroll
-                    for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(from_fixed32(v[k] + 1, 0));
+                    for (int k = 0; k < CPT; ++k) nxt[k] = as_dbl(whole_bits((v[k] >> iw_fin.shift) + iw_fin.add + 1));  // below 2^20
                     done = true;
                 }
             }
@@ -1668,13 +1985,6 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
     }
 }
 
-#ifndef PRK_STRICT_BLOCKS_1
-#define PRK_STRICT_BLOCKS_1 3
-#endif
-#ifndef PRK_STRICT_BLOCKS_N
-#define PRK_STRICT_BLOCKS_N 3
-#endif
-
 // Register budget: the single-application kernels keep as many tiles resident as shared memory
 // allows, so that every SM has enough loads in flight; the multi-application kernels hold `out` in
 // registers and run at most four tiles per SM. The strict FP64 form is bound by the binary64 pipe
@@ -1682,13 +1992,13 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
 template <int P, int R, int DT, int STEPS, int TH_>
 constexpr int min_blocks()
 {
-    // the table route: three tiles per SM (80 registers), so that 24 warps hide the fixed-point
-    // chains' latencies (at four, 64 registers, the longer chains spill); tiles whose shared memory
-    // (tile and tables) admits at most two per SM get the registers of two (the 64-row tiles of grid
-    // R=3..5: at three, grid R=5 spilled 3 KB)
+    // the table route: as many 32-row tiles as strict_tiles says (n=8192, four against three: star R=3 686
+    // us per application against 765, its whole runs 430 against 463; grid R=2 865 against 937); tiles
+    // whose shared memory admits at most two per SM get the registers of two (the 64-row tiles of grid
+    // R=3..5)
     if (DT == FP64 && !pow2_weights(P, R)) {
-        if (SMEM_PER_SM / (tile_smem<P, R, DT, TH_>() + 1024) < 3) return 2;
-        return one_application(STEPS) ? PRK_STRICT_BLOCKS_1 : PRK_STRICT_BLOCKS_N;
+        constexpr int fit = SMEM_PER_SM / (tile_smem<P, R, DT, TH_>() + 1024);
+        return fit < 3 ? 2 : (fit < strict_tiles<P, R>() ? fit : strict_tiles<P, R>());
     }
     if (DT == FP32C && P == GRID && R >= 3) return 2;  // bound by FP32 issue: registers over residency
     const int b = Geo<DT, R, TH_>::CTAS;

@@ -87,7 +87,7 @@ int table_route_split(int pattern, int R, int depth, int* fixed_adds, int* binar
 #define PRK_SPLIT(PP, RR)                                                                            \
     if (pattern == PP && R == RR) {                                                                  \
         if constexpr (tile::table_route<PP, RR, FP64>()) {                                            \
-            kf = depth == 1 ? tile::fixed_taps<PP, RR, true>() : tile::fixed_taps<PP, RR, false>();    \
+            kf = depth == 1 ? tile::narrow_taps<PP, RR, true>() : tile::narrow_taps<PP, RR, false>();  \
             n = tap_count(PP, RR);                                                                    \
         }                                                                                             \
     }
