@@ -91,12 +91,16 @@ struct Layout {
 };
 
 // Stage the `in` tile at (i0, j0) with its halo in shared memory: coalesced plain loads, zero
-// outside the arrays (nr rows of n columns), all loads issued before the first shared-memory store. Thread t takes elements
-// t, t + THREADS, ... of the row-major tile; its row, column and grid offset advance by constants
-// from one element to the next (one division per thread, none per element).
-template <int R, int DT>
-__device__ __forceinline__ void stage_tile(unsigned char* smem, const void* in_v, int64_t n, int64_t nr, int64_t i0,
-                                           int64_t j0)
+// outside the arrays (nr rows of n columns), all loads issued before the first shared-memory store.
+// Thread t takes elements t, t + THREADS, ... of the row-major tile; its row, column and grid offset
+// advance by constants from one element to the next (one division per thread, none per element).
+// FP32C: the values are checked for the integer route (tile::IntTile) on their way from the registers
+// and stored as that route wants them, or as they are when some value fails; the barrier that ends the
+// staging collects the verdict, so the check adds no pass over the tile and no barrier. row_hi: the first
+// array row no point reads.
+template <int P, int R, int DT, int STEPS>
+__device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const void* in_v, int64_t n, int64_t nr,
+                                                    int64_t i0, int64_t j0, int64_t row_hi, int nsteps)
 {
     using G = tile::Geo<DT, R>;
     using T = typename tile::Cfg<DT>::T;
@@ -108,12 +112,22 @@ __device__ __forceinline__ void stage_tile(unsigned char* smem, const void* in_v
     int r = threadIdx.x / G::SW, c = threadIdx.x - (threadIdx.x / G::SW) * G::SW;
     int gi = static_cast<int>(i0) - R + r, gj = static_cast<int>(j0) - G::RA + c;
     int64_t off = static_cast<int64_t>(gi) * n + gj;
+    tile::IntTile it;
+    constexpr bool CHECK = tile::int_route<P, R, DT, STEPS, true>();
+    if constexpr (CHECK) {  // the value nearest the tile's middle inside the grid
+        const int64_t rm = min(i0 - R + G::SH / 2, row_hi - 1), cm = min(j0 - G::RA + G::SW / 2, n - 1);
+        it.ref = in[rm * n + cm];
+    }
     T v[PER];
+    uint32_t loaded = 0;
+    static_assert(PER <= 32, "one bit per element of a thread");
 #pragma unroll
     for (int q = 0; q < PER; ++q) {  // all loads first, then the shared-memory stores
         const int idx = threadIdx.x + q * tile::THREADS;
-        const bool ok = (q + 1) * tile::THREADS <= G::ELEMS || idx < G::ELEMS;
-        v[q] = (ok && static_cast<uint32_t>(gi) < unr && static_cast<uint32_t>(gj) < un) ? in[off] : T(0);
+        const bool ok = ((q + 1) * tile::THREADS <= G::ELEMS || idx < G::ELEMS) && static_cast<uint32_t>(gi) < unr &&
+                        static_cast<uint32_t>(gj) < un;
+        v[q] = ok ? in[off] : T(0);
+        if (CHECK && ok) loaded |= 1u << q;
         c += DC;
         gi += DR;
         gj += DC;
@@ -125,12 +139,36 @@ __device__ __forceinline__ void stage_tile(unsigned char* smem, const void* in_v
             off += n - G::SW;
         }
     }
+    auto store = [&](auto f) {
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int idx = threadIdx.x + q * tile::THREADS;
-        if (idx < G::ELEMS) s_in[idx] = v[q];
+        for (int q = 0; q < PER; ++q) {
+            const int idx = threadIdx.x + q * tile::THREADS;
+            if (idx < G::ELEMS) s_in[idx] = f(q);
+        }
+    };
+    if constexpr (CHECK) {
+        tile::IntCheck check;
+        if (i0 >= R && j0 >= G::RA && i0 - R + G::SH <= nr && j0 - G::RA + G::SW <= n) {  // every element loaded
+            store([&](int q) {
+                const float u = __fsub_rn(v[q], it.ref);
+                if ((q + 1) * tile::THREADS <= G::ELEMS || threadIdx.x + q * tile::THREADS < G::ELEMS) check.add(u);
+                return u;
+            });
+        } else {
+            store([&](int q) {
+                const float u = __fsub_rn(v[q], it.ref);
+                if (loaded >> q & 1u) check.add(u);
+                return u;
+            });
+        }
+        it.known = true;
+        it.sums = check.sums<P, R>(it.ref, nsteps);
+        if (it.sums) return it;
+        it.ref = 0.0f;
     }
+    store([&](int q) { return v[q]; });
     __syncthreads();
+    return it;
 }
 
 // One work item: load the tile of grid g at `parity`, then evaluate it. tbl: the table area.
@@ -146,10 +184,11 @@ __device__ __forceinline__ void item(unsigned char* smem, int* s_red, const Grid
     // local memory)
     void* const in_cur = parity ? g.in[1] : g.in[0];
     void* const in_nxt = parity ? g.in[0] : g.in[1];
-    stage_tile<R, DT>(smem, in_cur, n, n, i0, j0);
+    const int nsteps = STEPS > 0 ? STEPS : depth;
+    const tile::IntTile it = stage_tile<P, R, DT, STEPS>(smem, in_cur, n, n, i0, j0, n, nsteps);
     tile::process_tile<P, R, DT, STEPS, tile::OUT_HBM>(smem, s_red, i0, j0, n, tile::tile_has_out(i0, j0, n, R, C::TW, C::TH),
                                                in_nxt, g.out, g.vec_ok != 0, depth, 0, n,
-                                               tile::table_route<P, R, DT>() ? tbl : nullptr);
+                                               tile::table_route<P, R, DT>() ? tbl : nullptr, it);
 }
 
 template <int DT, int STEPS, int FAM>

@@ -31,6 +31,8 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "prk_arith.cuh"
 #include "prk_fixed.cuh"
 #include "prk_internal.cuh"
@@ -338,6 +340,181 @@ __device__ __forceinline__ void fp32c_taps(const float* s, int ld, float (&sh)[C
             }
         }
     }
+}
+
+// ---------------------------------------------------------------------------------------------
+// FP32C, the integer route. Every PRK weight is +-1/den, so with M the common denominator of a
+// stencil M * S is a sum of integer coefficients times values. On a tile of whole numbers within B of
+// one another that sum is an integer small enough for FP32 arithmetic to be exact in any order, so the
+// taps cost one FMA each and the division by M, with its remainder, comes once, after every application
+// of the launch has been summed: no TwoSum and no split-weight products per group and application, and
+// a smaller error (one division's). The tile holds u = in - ref, ref a value of the tile, to keep the
+// partial sums small; in += 1 advances u. A thread's rows share every row segment it reads.
+// Bound by the FMA pipe (grid R >= 3) and by shared memory (about 28 bytes per point and application);
+// the group sums were bound by FP32 issue (star R=4, eight applications: FMA pipe 68%, issue 78%). At
+// n=8192, us per application of whole runs of 16, before and after: star R=2 87 to 51, star R=4 138 to
+// 61, star R=5 171 to 78, grid R=3 262 to 100, grid R=5 502 to 222; one application, grid R=5 591 to 420.
+
+__host__ __device__ constexpr int gcd_of(int a, int b) { return b == 0 ? a : gcd_of(b, a % b); }
+
+// Common denominator M of the weights.
+template <int P, int R>
+__host__ __device__ constexpr int common_den()
+{
+    int m = 1;
+    for (int dc = -R; dc <= R; ++dc)
+        for (int dr = -R; dr <= R; ++dr) {
+            const int d = weight_den(P, R, dc, dr);
+            if (d != 0) m = m / gcd_of(m, d) * d;
+        }
+    return m;
+}
+
+// M * weight of every tap, c[R + dr][R + dc]. A table made at compile time: evaluated per tap in the
+// unrolled loops, the weights' divisions stayed in the code of some stencils.
+template <int P, int R>
+struct IntCoefs {
+    int c[2 * R + 1][2 * R + 1];
+    int l1;
+};
+
+template <int P, int R>
+__host__ __device__ constexpr IntCoefs<P, R> make_int_coefs()
+{
+    IntCoefs<P, R> t{};
+    for (int dc = -R; dc <= R; ++dc)
+        for (int dr = -R; dr <= R; ++dr) {
+            const int d = weight_den(P, R, dc, dr);
+            if (d == 0) continue;
+            t.c[R + dr][R + dc] = weight_sign(P, R, dc, dr) * (common_den<P, R>() / d);
+            t.l1 += common_den<P, R>() / d;
+        }
+    return t;
+}
+
+// Range of the tile's values, |u| < B at the launch's first application: 128, which a PRK field's tiles
+// keep (their values lie within 110 of the middle one), or the stencil's largest.
+constexpr int INT_NEAR = 128;
+
+template <int P, int R>
+__host__ __device__ constexpr int int_wide()
+{
+    int b = INT_NEAR;
+    while (b < (1 << 17) && static_cast<int64_t>(8) * b * make_int_coefs<P, R>().l1 < (1 << 24)) b *= 2;
+    return b;
+}
+
+// Applications whose sums one FP32 accumulator takes, and applications a launch may make on the route.
+// An application's M * S is at most L1 (B - 1) (its taps in pairs of opposite weight, each difference at
+// most 2 (B - 1)); while it forms, its partial sums reach L1 (B + t) for |u| < B + t. Together they stay
+// below 2^24 for SUMS applications in a row and STEPS in all, and the sum over STEPS below 2^31.
+template <int P, int R, int B>
+struct IntBound {
+    static constexpr int64_t L1 = make_int_coefs<P, R>().l1, LIMIT = (1 << 24) - 1;
+    static constexpr int64_t MAX_S = L1 * (B - 1);
+    static constexpr int64_t SUMS0 = LIMIT / 2 / MAX_S + 1;
+    static constexpr int SUMS = static_cast<int>(SUMS0 > 16 ? 16 : SUMS0);
+    static constexpr int64_t STEPS0 = (LIMIT - (SUMS - 1) * MAX_S) / L1 - B;
+    static constexpr int64_t STEPS1 = ((1ll << 31) - 1) / MAX_S;
+    static constexpr int STEPS = static_cast<int>(STEPS0 < STEPS1 ? STEPS0 : STEPS1);
+    static_assert(SUMS >= 1 && STEPS >= INT_NEAR && STEPS + B < (1 << 23),
+                  "integer route bounds");
+};
+
+// Launches that try the integer route: all on the TMA tiles (PLAIN false), where one fused application
+// is bound by HBM on either route and grid R >= 3 gains (n=8192, grid R=4: 419 to 327 us), so that a
+// result does not depend on the depth. On the plain-staged tiles, bound by issue, one fused application
+// of the others keeps the group sums (n=8189, star R=1: 274 us; 307 with the check while staging).
+template <int P, int R, int DT, int STEPS, bool PLAIN>
+__host__ __device__ constexpr bool int_route()
+{
+    return DT == FP32C && (!PLAIN || STEPS != 1 || (P == GRID && R >= 3));
+}
+
+// Whether a staged FP32C tile takes the integer route, and its ref: checked while it was staged by plain
+// loads (known), or to be checked in the evaluation. sums: IntBound::SUMS of its range, 0 off the route.
+struct IntTile {
+    bool known = false;
+    int sums = 0;
+    float ref = 0.0f;
+};
+
+// |x| < 2^22 and whole.
+__device__ __forceinline__ bool whole_f32(float x) { return __fsub_rn(__fadd_rn(x, 12582912.0f), 12582912.0f) == x; }
+
+// The tile's values u = in - ref: whole, and the largest |u|. in is then whole, as ref is.
+struct IntCheck {
+    bool whole = true;
+    float most = 0.0f;
+    __device__ __forceinline__ void add(float u)
+    {
+        whole = whole && whole_f32(u);
+        most = fmaxf(most, fabsf(u));
+    }
+    // The block's verdict (a barrier, or two where the values are not near): IntTile::sums.
+    template <int P, int R>
+    __device__ __forceinline__ int sums(float ref, int nsteps) const
+    {
+        using Near = IntBound<P, R, INT_NEAR>;
+        using Wide = IntBound<P, R, int_wide<P, R>()>;
+        const bool ok = whole && fabsf(ref) < 8388608.0f && rintf(ref) == ref;  // in + steps below 2^24
+        if (__syncthreads_and(ok && most < static_cast<float>(INT_NEAR) && nsteps <= Near::STEPS)) return Near::SUMS;
+        if (int_wide<P, R>() > INT_NEAR &&
+            __syncthreads_and(ok && most < static_cast<float>(int_wide<P, R>()) && nsteps <= Wide::STEPS))
+            return Wide::SUMS;
+        return 0;
+    }
+};
+
+// S[rr][k] += M * S of the thread's CPT points of ROWS consecutive rows; u points at (r0, c0) of the tile.
+// Row by row of the tile: each row segment is read once and enters every output row it is a tap of.
+template <int P, int R, int CPT, int ROWS, int RA>
+__device__ __forceinline__ void int_rows(const float* u, int ld, float (&S)[ROWS][CPT])
+{
+    constexpr IntCoefs<P, R> C = make_int_coefs<P, R>();
+#pragma unroll
+    for (int q = -R; q < ROWS + R; ++q) {
+        auto taps = [&](auto pad, const auto& seg) {
+            constexpr int PAD = decltype(pad)::value;
+#pragma unroll
+            for (int rr = 0; rr < ROWS; ++rr) {
+                const int dr = q - rr;
+#pragma unroll
+                for (int dc = -PAD; dc <= PAD; ++dc) {
+                    const int c = dr >= -R && dr <= R && dc >= -R && dc <= R ? C.c[R + dr][R + dc] : 0;
+                    if (c != 0) {
+#pragma unroll
+                        for (int k = 0; k < CPT; ++k)
+                            S[rr][k] = __fmaf_rn(static_cast<float>(c), seg[k + PAD + dc], S[rr][k]);
+                    }
+                }
+            }
+        };
+        if (P == GRID || (q >= 0 && q < ROWS)) {
+            float seg[CPT + 2 * RA];
+            ld_seg<CPT + 2 * RA>(u + q * ld - RA, seg);
+            taps(std::integral_constant<int, RA>{}, seg);
+        } else {  // star: a row above or below the thread's is a vertical tap only
+            float seg[CPT];
+            ld_seg<CPT>(u + q * ld, seg);
+            taps(std::integral_constant<int, 0>{}, seg);
+        }
+    }
+}
+
+// (o_hi, o_lo) += (t + tl) / M, renormalised, for whole t and tl (t a float's 24 bits, |tl| far smaller):
+// q near t / M, the remainder t - q M exact (a small multiple of q's last bit), and the remainder's share
+// of the quotient as the low word. Exact where M divides t, as it does for a PRK field.
+template <int P, int R>
+__device__ __forceinline__ void int_add(uint64_t& o, float t, float tl)
+{
+    constexpr int M = common_den<P, R>();
+    constexpr float INV = static_cast<float>(1.0 / M);
+    const float q = __fmul_rn(t, INV);
+    const float rem = __fmaf_rn(-q, static_cast<float>(M), t);
+    float oh = __uint_as_float(static_cast<uint32_t>(o)), ol = __uint_as_float(static_cast<uint32_t>(o >> 32));
+    df_add(oh, ol, q, __fmul_rn(__fadd_rn(rem, tl), INV));
+    o = static_cast<uint64_t>(__float_as_uint(oh)) | (static_cast<uint64_t>(__float_as_uint(ol)) << 32);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1405,7 +1582,7 @@ template <int P, int R, int DT, int STEPS, int OUT_SRC = OUT_SMEM, int TH_ = 32>
 __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, int64_t i0, int64_t j0, int64_t n,
                                              bool has_out, void* __restrict__ in_next_v, void* __restrict__ out_v,
                                              bool vec_ok, int depth, int64_t goff, int64_t row_end,
-                                             unsigned char* tbl)
+                                             unsigned char* tbl, const IntTile& pre = IntTile{})
 {
     const int nsteps = STEPS > 0 ? STEPS : (STEPS == OPERATOR ? 1 : depth);
     using G = Geo<DT, R, TH_>;
@@ -1522,6 +1699,17 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         }
         __syncthreads();  // every converted word visible
     }
+    // Elements no stored point reads (outside the grid, or past the last row's halo) hold zeros. They stay
+    // out of a tile's range, so that a tile at the grid's edge has the range of its own values: counted
+    // in, they made it too wide for the table and integer routes (at n=1000 on 18% of the tiles).
+    const int64_t row_hi = min(row_end + R, n - goff);  // first array row past those that are read
+    const bool edge = i0 < R || j0 < G::RA || i0 + C::TH + R > row_hi || j0 + C::TW + G::RA > n;
+    auto inside = [&](int idx) {
+        const int r = idx / G::SW, c = idx - r * G::SW;
+        return static_cast<uint64_t>(i0 - R + r) < static_cast<uint64_t>(row_hi) &&
+               static_cast<uint64_t>(j0 - G::RA + c) < static_cast<uint64_t>(n);
+    };
+
     // ---- FP64, other weights: whole-number tiles take their products off the binary64 pipe ----
     // Every value +0 or a whole number below 2^19 (so that up to 2^19 applications of in += 1 stay
     // below 2^20): the tile is held as int32 and fp64_points_whole evaluates it.
@@ -1531,17 +1719,6 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         const uint64_t* raw = reinterpret_cast<const uint64_t*>(s_in);
         int32_t iv[PER];
         bool ok = nsteps <= (1 << 19);
-        // Elements no stored point reads (outside the grid, or past the last row's halo) hold zeros; they
-        // stay out of the tile's range and take its lowest value, so that a tile at the grid's edge has
-        // the range of its own values. (Its halo's zeros made the range too wide for the tables: at
-        // n=1000 18% of the tiles took the product route for it.)
-        const int64_t row_hi = min(row_end + R, n - goff);  // first array row past those that are read
-        const bool edge = i0 < R || j0 < G::RA || i0 + C::TH + R > row_hi || j0 + C::TW + G::RA > n;
-        auto inside = [&](int idx) {
-            const int r = idx / G::SW, c = idx - r * G::SW;
-            return static_cast<uint64_t>(i0 - R + r) < static_cast<uint64_t>(row_hi) &&
-                   static_cast<uint64_t>(j0 - G::RA + c) < static_cast<uint64_t>(n);
-        };
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
             const int idx = threadIdx.x + q * THREADS;
@@ -1617,29 +1794,46 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
     // The table route with out in HBM has stored out itself; the stores then write in_next only
     const bool out_via_rows = !(tbl_done && OUT_SRC != OUT_SMEM);
 
-    // ---- FP32C, the operator form: one compensated product per tap, or per weight group ----
-    // fp32c_points sums a weight group's differences before the product, which is exact for whole
-    // numbers near one another but rounds once per tap for others; the operator form takes the
-    // per-tap products (fp32c_taps) there. A tile takes the group sums when every value is a whole
-    // number below 2^22 within 2^18 of the tile's first: its differences stay below 2^19 and a
-    // group's sum of at most 18 of them (grid R=5, sides of ring 5) below 2^24.
-    bool grouped = true;
-    if constexpr (DT == FP32C && STEPS == OPERATOR) {
-        constexpr int NV = G::ELEMS / 4;
-        static_assert(G::ELEMS % 4 == 0, "the check reads 16-byte vectors");
-        const float ref = s_in[R * G::SW + G::RA];
-        bool ok = true;
-        for (int idx = threadIdx.x; idx < NV; idx += THREADS) {
-            const float4 v = reinterpret_cast<const float4*>(s_in)[idx];
-            const float e[4] = {v.x, v.y, v.z, v.w};
+    // ---- FP32C: whole-number tiles of small range take the integer route ----
+    int sums = 0;  // applications one FP32 sum takes on the route
+    float uref = 0.0f;
+    if constexpr (int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>()) {
+        if (pre.known) {
+            sums = pre.sums;
+            uref = pre.ref;
+        } else {
+            constexpr int NV = G::ELEMS / 4, PER = (NV + THREADS - 1) / THREADS;
+            static_assert(G::ELEMS % 4 == 0, "the tile as 16-byte vectors");
+            // the value nearest the tile's middle inside the grid
+            const int rm = static_cast<int>(min(static_cast<int64_t>(G::SH / 2), row_hi - 1 - (i0 - R)));
+            const int cm = static_cast<int>(min(static_cast<int64_t>(G::SW / 2), n - 1 - (j0 - G::RA)));
+            uref = s_in[rm * G::SW + cm];
+            float4 u[PER];
+            IntCheck check;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float whole = __fsub_rn(__fadd_rn(e[k], 12582912.0f), 12582912.0f);  // |e| < 2^22
-                ok = ok && fabsf(e[k]) < 4194304.0f && whole == e[k] && fabsf(__fsub_rn(e[k], ref)) < 262144.0f;
+            for (int q = 0; q < PER; ++q) {
+                const int v = threadIdx.x + q * THREADS;
+                u[q] = v < NV ? reinterpret_cast<const float4*>(s_in)[v] : make_float4(uref, uref, uref, uref);
+                float* e = reinterpret_cast<float*>(&u[q]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    e[k] = __fsub_rn(e[k], uref);
+                    if (!edge || inside(4 * v + k)) check.add(e[k]);
+                }
+            }
+            sums = check.sums<P, R>(uref, nsteps);
+            if (sums) {
+#pragma unroll
+                for (int q = 0; q < PER; ++q) {
+                    const int v = threadIdx.x + q * THREADS;
+                    if (v < NV) reinterpret_cast<float4*>(s_in)[v] = u[q];
+                }
+                __syncthreads();
             }
         }
-        grouped = __syncthreads_and(ok) != 0;
     }
+
+    const bool inted = sums != 0;
 
     // Set by the multi-application FP32 route when the tile's out words are held as integers
     bool oint = false;
@@ -1704,11 +1898,11 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         } else {
             const float* sp = reinterpret_cast<const float*>(s_in) + soff;
             float sh[CPT], sl[CPT];
-            if (grouped) {
+            // the operator form keeps one product per tap: a group's sum would round its differences again
+            if constexpr (STEPS == OPERATOR)
+                fp32c_taps<P, R, CPT, G::RA>(sp, G::SW, sh, sl);
+            else
                 fp32c_points<P, R, CPT, G::RA>(sp, G::SW, sh, sl);
-            } else {
-                if constexpr (STEPS == OPERATOR) fp32c_taps<P, R, CPT, G::RA>(sp, G::SW, sh, sl);
-            }
 #pragma unroll
             for (int k = 0; k < CPT; ++k) {
                 float oh = __uint_as_float(static_cast<uint32_t>(o[k]));
@@ -1761,8 +1955,8 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                 for (int k = 0; k < CPT; ++k) {
                     if constexpr (DT == FP64)
                         nxt[k] = inc_exact(s_in[soff + k]);
-                    else
-                        nxt[k] = __fadd_rn(s_in[soff + k], 1.0f);
+                    else  // the tile holds in - uref on the integer route
+                        nxt[k] = __fadd_rn(s_in[soff + k], inted ? __fadd_rn(uref, 1.0f) : 1.0f);
                 }
             }
             T* nx = static_cast<T*>(in_next_v) + gi * n + gj;
@@ -1809,6 +2003,11 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                 }
             }
         }
+        float si[int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>() ? ROWS : 1][CPT] = {};  // M * S of the thread's points (integer route)
+        if constexpr (int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>()) {
+            if (inted && has_out)
+                int_rows<P, R, CPT, ROWS, G::RA>(s_in + (warp * ROWS + R) * G::SW + G::RA + c0, G::SW, si);
+        }
 #pragma unroll
         for (int rr = 0; rr < ROWS; ++rr) {
             const int r = warp * ROWS + rr;
@@ -1823,13 +2022,68 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                 } else {
                     load_out_row(r, o);
                 }
-                if (!tbl_done) apply_row(r, o);
+                if constexpr (int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>()) {
+                    if (inted) {
+#pragma unroll
+                        for (int k = 0; k < CPT; ++k) int_add<P, R>(o[k], si[rr][k], 0.0f);
+                    }
+                }
+                if (!tbl_done && !inted) apply_row(r, o);
             }
             store_row(r, o, row_out);
         }
     } else {
-        // out of the thread's points stays in registers across the applications
         static_assert(G::ELEMS % 4 == 0, "the in-place advance moves 16-byte vectors");
+        if constexpr (DT == FP32C) {
+            if (inted) {
+                // The integer route: M * S of every application summed exactly, out read and updated once
+                // at the end. `sums` applications fit the FP32 sum; it then goes to an integer.
+                float a[ROWS][CPT] = {};
+                int acc[ROWS][CPT] = {};
+                int held = 0;
+#pragma unroll 1
+                for (int t = 0; t < nsteps; ++t) {
+                    if (t > 0) {
+                        __syncthreads();
+                        advance_f32<G::ELEMS>(s_in);
+                        __syncthreads();
+                    }
+                    if (held == sums) {
+                        held = 0;
+#pragma unroll
+                        for (int rr = 0; rr < ROWS; ++rr)
+#pragma unroll
+                            for (int k = 0; k < CPT; ++k) {
+                                acc[rr][k] += __float2int_rn(a[rr][k]);
+                                a[rr][k] = 0.0f;
+                            }
+                    }
+                    ++held;
+                    if (has_out)
+                        int_rows<P, R, CPT, ROWS, G::RA>(s_in + (warp * ROWS + R) * G::SW + G::RA + c0, G::SW, a);
+                }
+#pragma unroll
+                for (int rr = 0; rr < ROWS; ++rr) {
+                    const int r = warp * ROWS + rr;
+                    const int64_t gi = i0 + r, gg = gi + goff;
+                    if (!col_ok || gi >= row_end) continue;
+                    const bool row_out = has_out && gg >= R && gg < n - R;
+                    uint64_t o[CPT];
+                    if (row_out) {
+                        load_out_row(r, o);
+#pragma unroll
+                        for (int k = 0; k < CPT; ++k) {
+                            const int t = acc[rr][k] + __float2int_rn(a[rr][k]);
+                            const float th = __int2float_rn(t);
+                            int_add<P, R>(o[k], th, __int2float_rn(t - __float2int_rn(th)));
+                        }
+                    }
+                    store_row(r, o, row_out);
+                }
+                return;
+            }
+        }
+        // out of the thread's points stays in registers across the applications
         uint64_t o[ROWS][CPT];
         bool ract[ROWS];  // the row holds interior points
 #pragma unroll
@@ -2000,7 +2254,11 @@ constexpr int min_blocks()
         constexpr int fit = SMEM_PER_SM / (tile_smem<P, R, DT, TH_>() + 1024);
         return fit < 3 ? 2 : (fit < strict_tiles<P, R>() ? fit : strict_tiles<P, R>());
     }
-    if (DT == FP32C && P == GRID && R >= 3) return 2;  // bound by FP32 issue: registers over residency
+    // FP32C grid R >= 3: three tiles per SM (80 registers; n=8192, the integer route, us per application
+    // against two tiles: grid R=3 263 against 300 at one application, 100 against 105 in whole runs; R=5
+    // 420 against 446 and 222 against 228). The group sums of tiles off that route would want the
+    // registers of two.
+    if (DT == FP32C && P == GRID && R >= 3) return Geo<DT, R, TH_>::CTAS < 3 ? Geo<DT, R, TH_>::CTAS : 3;
     const int b = Geo<DT, R, TH_>::CTAS;
     if (one_application(STEPS)) return b;
     const int cap = DT == FP64 ? 4 : 3;  // FP64 power-of-two: the FP32 route is shared-memory bound

@@ -124,9 +124,11 @@ __global__ void __launch_bounds__(tile::THREADS, plain_min_blocks<P, R, DT, STEP
         tile::process_tile<P, R, DT, STEPS, tile::OUT_SMEM>(smem, s_red, i0, j0, n, has_out, in_next, out, false,
                                                             depth, goff, row_end, smem + S::TBL_OFF);
     } else {
-        batch::stage_tile<R, DT>(smem, in, n, nr, i0, j0);
+        const int nsteps = STEPS > 0 ? STEPS : (STEPS == tile::OPERATOR ? 1 : depth);
+        const int64_t row_hi = row_end + R < n - goff ? row_end + R : n - goff;  // past the rows that are read
+        const tile::IntTile it = batch::stage_tile<P, R, DT, STEPS>(smem, in, n, nr, i0, j0, row_hi, nsteps);
         tile::process_tile<P, R, DT, STEPS, tile::OUT_HBM_AHEAD>(smem, s_red, i0, j0, n, has_out, in_next, out,
-                                                                 false, depth, goff, row_end, nullptr);
+                                                                 false, depth, goff, row_end, nullptr, it);
     }
 }
 
