@@ -925,6 +925,28 @@ __device__ __forceinline__ void fp64_points_whole(const int32_t* s, double (&acc
     }
 }
 
+// The reference's chain with binary64 instructions throughout, for CPT adjacent points: the tiles no other
+// route takes (subnormals, infinities, NaNs and values near the ends of the exponent range). A loop over
+// the taps: it is bound by the binary64 pipe, and unrolled it cost the kernels around it registers.
+template <int P, int R, int LD, int CPT>
+__device__ __forceinline__ void fp64_points_strict(const double* s, double (&acc)[CPT])
+{
+    constexpr int N = tap_count(P, R);
+    const auto& T = c_taps<P, R, LD>;
+    auto weight_of = [](const auto& tp) {
+        return as_dbl((static_cast<uint64_t>(tp.hib | (tp.w2 & 0xFFFFFu)) << 32) | tp.w1);
+    };
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) acc[k] = __dmul_rn(s[T.tap[0].off + k], weight_of(T.tap[0]));
+#pragma unroll 1
+    for (int t = 1; t < N; ++t) {
+        const auto tp = T.tap[t];
+        const double w = weight_of(tp);
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) acc[k] = __dadd_rn(acc[k], __dmul_rn(s[tp.off + k], w));
+    }
+}
+
 // in += 1 over a staged tile of int32 whole numbers, as 16-byte vectors.
 template <int ELEMS>
 __device__ __forceinline__ void advance_i32(int32_t* p)
@@ -1400,6 +1422,180 @@ __device__ __forceinline__ void table_chain(const int32_t* sp, const unsigned ch
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// FP64, real-valued tiles: fewer binary64 instructions with the same roundings
+//
+// The binary64 pipe (1/73 of the FP32 rate) bounds a tile that no exact route takes: one rounded product
+// and one rounded add per tap. Two identities take most products off it without changing a bit, for
+// values that are zero or far from the ends of the exponent range (checked per tile):
+//  - Multiplying by +-2^-k is exact, so the product and the add of a power-of-two weight are one fused
+//    multiply-add.
+//  - fl(v / (2^k d)) = 2^-k fl(v / d), so the weights whose denominators share their odd part share one
+//    rounded product per value, and every tap that uses it is again a fused multiply-add by +-2^-k. The
+//    products of a family of weights are computed once per value into a plane of the tile in shared
+//    memory (of `out` words and tables that this path does not need by then) instead of once per tap.
+// A family that has no plane multiplies per tap. Binary64 instructions per point, before and now: star
+// R=2 17 and 10, star R=3 24 and 16, grid R=2 37 and 23. At n=8192, one fused application, us: star R=2
+// 2185 to 1293, R=3 3199 to 2019, R=4 4215 to 2493, R=5 5229 to 3907; grid R=2 4850 to 2974, R=3 9926 to
+// 8071, R=4 16775 to 13154, R=5 25399 to 22047.
+
+__host__ __device__ constexpr int odd_part(int d)
+{
+    while (d % 2 == 0) d /= 2;
+    return d;
+}
+
+// The families of a stencil: plane 0 is the tile itself (family 1, weights that are powers of two) or, in
+// place of it, the plane of a family; plane 1 the family with the most taps beside it (0: none).
+template <int P, int R, bool INPLACE>
+struct RealPlan {
+    int fam0 = 1, fam1 = 0;        // odd parts
+    int den0 = 1, den1 = 1;        // the planes hold fl(v / den)
+    int off_dr[tap_count(P, R)] = {}, off_dc[tap_count(P, R)] = {};
+    int plane[tap_count(P, R)] = {};   // 0, 1, or 2: a product of its own
+    double c[tap_count(P, R)] = {};    // the factor of the plane's value, or the weight
+};
+
+template <int P, int R>
+__host__ __device__ constexpr int taps_of_family(int fam)
+{
+    int k = 0;
+    for (int dc = -R; dc <= R; ++dc)
+        for (int dr = -R; dr <= R; ++dr) {
+            const int d = weight_den(P, R, dc, dr);
+            if (d != 0 && odd_part(d) == fam) ++k;
+        }
+    return k;
+}
+
+// The family with the most taps other than 1 and `but`, 0 when there is none.
+template <int P, int R>
+__host__ __device__ constexpr int largest_family(int but)
+{
+    int best = 0, most = 0;
+    for (int dc = -R; dc <= R; ++dc)
+        for (int dr = -R; dr <= R; ++dr) {
+            const int d = weight_den(P, R, dc, dr);
+            if (d == 0) continue;
+            const int f = odd_part(d);
+            if (f != 1 && f != but && taps_of_family<P, R>(f) > most) {
+                best = f;
+                most = taps_of_family<P, R>(f);
+            }
+        }
+    return best;
+}
+
+// True when two families cover every tap, so that both planes' values replace the tile's.
+template <int P, int R>
+__host__ __device__ constexpr bool two_families()
+{
+    const int a = largest_family<P, R>(0);
+    const int b = a ? largest_family<P, R>(a) : 0;
+    return b != 0 && taps_of_family<P, R>(a) + taps_of_family<P, R>(b) == tap_count(P, R);
+}
+
+template <int P, int R, bool INPLACE>
+constexpr RealPlan<P, R, INPLACE> make_real_plan()
+{
+    RealPlan<P, R, INPLACE> t{};
+    const int big = largest_family<P, R>(0);
+    if (INPLACE) {
+        t.fam0 = big;
+        t.fam1 = largest_family<P, R>(big);
+    } else {
+        t.fam1 = big;
+    }
+    // a plane's denominator: the first tap's of its family, so that the chain's first product needs no factor
+    for (int pass = 0; pass < 2; ++pass) {
+        int k = 0;
+        bool set0 = false, set1 = false;
+        for (int dc = -R; dc <= R; ++dc)
+            for (int dr = -R; dr <= R; ++dr) {
+                const int d = weight_den(P, R, dc, dr);
+                if (d == 0) continue;
+                const int f = odd_part(d), s = weight_sign(P, R, dc, dr);
+                if (pass == 0) {
+                    if (INPLACE && f == t.fam0 && !set0) {
+                        t.den0 = d;
+                        set0 = true;
+                    }
+                    if (t.fam1 != 0 && f == t.fam1 && !set1) {
+                        t.den1 = d;
+                        set1 = true;
+                    }
+                } else {
+                    t.off_dr[k] = dr;
+                    t.off_dc[k] = dc;
+                    t.plane[k] = f == t.fam0 ? 0 : (f == t.fam1 ? 1 : 2);
+                    const int den = t.plane[k] == 0 ? t.den0 : t.den1;
+                    t.c[k] = t.plane[k] == 2 ? weight(P, R, dc, dr) : s * (static_cast<double>(den) / d);
+                }
+                ++k;
+            }
+    }
+    return t;
+}
+
+// The planes of the staged tile: plane 1 beside it, and plane 0 in its place (INPLACE).
+template <int P, int R, bool INPLACE, int ELEMS>
+__device__ __forceinline__ void real_planes(double* s_in, double* p1)
+{
+    constexpr RealPlan<P, R, INPLACE> T = make_real_plan<P, R, INPLACE>();
+    if constexpr (T.fam1 != 0) {
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < ELEMS; idx += THREADS) {
+            const double v = s_in[idx];
+            p1[idx] = __dmul_rn(v, 1.0 / T.den1);
+            if (INPLACE) s_in[idx] = __dmul_rn(v, 1.0 / T.den0);
+        }
+    }
+}
+
+// S of CPT adjacent points: the reference's chain, its products from the planes; p0 and p1 point at the
+// first point's value in them.
+template <int P, int R, bool INPLACE, int LD, int CPT>
+__device__ __forceinline__ void real_points(const double* p0, const double* p1, double (&acc)[CPT])
+{
+    constexpr RealPlan<P, R, INPLACE> T = make_real_plan<P, R, INPLACE>();
+#pragma unroll
+    for (int t = 0; t < tap_count(P, R); ++t) {
+        const double* src = (T.plane[t] == 1 ? p1 : p0) + T.off_dr[t] * LD + T.off_dc[t];
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) {
+            if (t == 0)
+                acc[k] = T.c[t] == 1.0 && T.plane[t] != 2 ? src[k]
+                         : T.c[t] == -1.0 && T.plane[t] != 2
+                             ? as_dbl(as_bits(src[k]) ^ fx::SIGN)
+                             : __dmul_rn(src[k], T.c[t]);
+            else if (T.plane[t] == 2)
+                acc[k] = __dadd_rn(acc[k], __dmul_rn(src[k], T.c[t]));
+            else
+                acc[k] = __fma_rn(src[k], T.c[t], acc[k]);
+        }
+    }
+}
+
+// S of two adjacent points, by real_points (real) or fp64_points_strict. A call, so that its registers are
+// its own: inlined, it spilled the HBM-bound kernels around it (n=16384, one fused application, star R=2
+// 1209 us against 1205); bound by the binary64 pipe, it loses nothing by it.
+template <int P, int R, bool INPLACE, int LD>
+__device__ __noinline__ double2 fp64_pair(const double* p0, const double* p1, bool real)
+{
+    double d[2];
+    if (real)
+        real_points<P, R, INPLACE, LD, 2>(p0, p1, d);
+    else
+        fp64_points_strict<P, R, LD, 2>(p0, d);
+    return make_double2(d[0], d[1]);
+}
+
+// A value the path takes: zero, or normal with every product of it normal.
+__device__ __forceinline__ bool real_value(uint64_t b)
+{
+    return (b << 1) == 0 || ((static_cast<uint32_t>(b >> 52) & 0x7FFu) - 128u) < 1772u;
+}
+
 // Bytes of the shared-memory out area the table route needs besides its tables in kernels that keep
 // out in HBM (one FP64 tile of out words; the TMA kernel updates its out tile instead).
 __host__ __device__ constexpr int table_out_bytes() { return Cfg<FP64>::TW * Cfg<FP64>::TH * 8; }
@@ -1835,6 +2031,35 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
 
     const bool inted = sums != 0;
 
+    // ---- FP64, real-valued tiles: products shared or fused into the adds (real_points) ----
+    constexpr bool INPLACE = one_application(STEPS) && two_families<P, R>();
+    constexpr bool PLANES = DT == FP64 && !EXACT;  // the power-of-two stencils need no plane beside the tile
+    bool real = false;
+    double* p1 = nullptr;  // plane 1: over the out words (read into registers first) and the tables
+    if constexpr (DT == FP64) {
+        if ((EXACT ? one_application(STEPS) && !fexact && unit == fx::NOT_FIXED : !iwhole) && (!PLANES || tbl)) {
+            bool ok = true;
+            for (int idx = threadIdx.x; idx < G::ELEMS; idx += THREADS)
+                ok = ok && real_value(reinterpret_cast<const uint64_t*>(s_in)[idx]);
+            real = __syncthreads_and(ok) != 0;
+            p1 = reinterpret_cast<double*>(OUT_SRC == OUT_SMEM ? stage + G::OUT_OFF : tbl);
+            constexpr int AREA = OUT_SRC == OUT_SMEM
+                                     ? table_offset<DT, R, TH_>() + table_bytes<P, R, DT>() - G::OUT_OFF
+                                     : table_bytes<P, R, DT>() + table_out_bytes();
+            static_assert(!PLANES || AREA >= G::IN_BYTES, "plane 1 fits over the out words and the tables");
+        }
+    }
+    // S of the two points of row r by binary64 instructions, into the out words
+    auto fp64_row = [&](int r, uint64_t* o) {
+        if constexpr (DT == FP64) {
+            const int soff = (r + R) * G::SW + G::RA + c0;
+            const double2 S =
+                fp64_pair<P, R, INPLACE, G::SW>(reinterpret_cast<const double*>(s_in) + soff, p1 + soff, real);
+            o[0] = as_bits(__dadd_rn(as_dbl(o[0]), S.x));
+            o[1] = as_bits(__dadd_rn(as_dbl(o[1]), S.y));
+        }
+    };
+
     // Set by the multi-application FP32 route when the tile's out words are held as integers
     bool oint = false;
     // Offset in floats of the FP32 tile holding the last application's in (double-buffered route)
@@ -1890,10 +2115,16 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                     done = true;
                 }
             }
-            if (!done) {
-                const double* sp = reinterpret_cast<const double*>(s_in) + soff;
+            if constexpr (EXACT && !one_application(STEPS)) {
+                // products and adds apart, inlined: calls here cost the FP32 loop of several applications 2%
+                if (!done) {
+                    const double* sp = reinterpret_cast<const double*>(s_in) + soff;
 #pragma unroll
-                for (int k = 0; k < CPT; ++k) o[k] = as_bits(__dadd_rn(as_dbl(o[k]), fp64_point<P, R>(sp + k, G::SW)));
+                    for (int k = 0; k < CPT; ++k)
+                        o[k] = as_bits(__dadd_rn(as_dbl(o[k]), fp64_point<P, R>(sp + k, G::SW)));
+                }
+            } else if (!done) {
+                fp64_row(r, o);
             }
         } else {
             const float* sp = reinterpret_cast<const float*>(s_in) + soff;
@@ -1916,10 +2147,10 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         }
     };
 
-    // in_next (in + 1 after the last application) and out of row r to HBM
-    auto store_row = [&](int r, const uint64_t* o, bool row_out) {
-        const int64_t gi = i0 + r;
+    // in_next (in + 1 after the last application) of row r to HBM
+    auto store_next = [&](int r) {
         if constexpr (STEPS != OPERATOR) {
+            const int64_t gi = i0 + r;
             const int soff = (r + R) * G::SW + G::RA + c0;
             T nxt[CPT];
             bool done = false;
@@ -1970,6 +2201,11 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                     if (gj + k < n) nx[k] = nxt[k];
             }
         }
+    };
+
+    // and out
+    auto store_out = [&](int r, const uint64_t* o, bool row_out) {
+        const int64_t gi = i0 + r;
         if (row_out) {
             uint64_t* out = static_cast<uint64_t*>(out_v) + gi * n + gj;
             if (cols_interior && (vec_ok || (reinterpret_cast<uintptr_t>(out) & 15u) == 0)) {
@@ -1983,6 +2219,58 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         }
     };
 
+    auto store_row = [&](int r, const uint64_t* o, bool row_out) {
+        store_next(r);
+        store_out(r, o, row_out);
+    };
+
+    if constexpr (one_application(STEPS) && PLANES) {
+        if (real) {
+            // in_next leaves first (the tile may be overwritten by a plane), and out waits in registers
+            uint64_t o[ROWS][CPT];
+            bool act[ROWS];
+#pragma unroll
+            for (int rr = 0; rr < ROWS; ++rr) {
+                const int r = warp * ROWS + rr;
+                const int64_t gi = i0 + r, gg = gi + goff;
+                const bool row = col_ok && gi < row_end;
+                act[rr] = row && has_out && gg >= R && gg < n - R;
+                if (row) store_next(r);
+                if (act[rr]) load_out_row(r, o[rr]);
+            }
+            __syncthreads();  // every thread has read its values and out words
+            real_planes<P, R, INPLACE, G::ELEMS>(reinterpret_cast<double*>(s_in), p1);
+            __syncthreads();
+#pragma unroll
+            for (int rr = 0; rr < ROWS; ++rr) {
+                const int r = warp * ROWS + rr;
+                if (!act[rr]) continue;
+                fp64_row(r, o[rr]);
+                store_out(r, o[rr], true);
+            }
+            return;
+        }
+    }
+    if constexpr (one_application(STEPS) && EXACT) {
+        if (!fexact) {
+            // the other routes row by row in a loop of their own, so that the FP32 route's code below keeps
+            // its registers
+#pragma unroll 1
+            for (int rr = 0; rr < ROWS; ++rr) {
+                const int r = warp * ROWS + rr;
+                const int64_t gi = i0 + r, gg = gi + goff;
+                if (!col_ok || gi >= row_end) continue;
+                const bool row_out = has_out && gg >= R && gg < n - R;
+                uint64_t o[CPT];
+                if (row_out) {
+                    load_out_row(r, o);
+                    apply_row(r, o);
+                }
+                store_row(r, o, row_out);
+            }
+            return;
+        }
+    }
     if constexpr (one_application(STEPS)) {
         // one pass: each row's new out and in_next leave as soon as they are computed. OUT_HBM_AHEAD:
         // every row's out words are requested first, so that their latencies overlap instead of
@@ -2200,6 +2488,17 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                     advance_f32<G::ELEMS>(s_in);
                 }
                 __syncthreads();
+            }
+            if constexpr (PLANES) {
+                if (real) {
+                    if (t == 0) __syncthreads();  // every thread has its out words in registers
+                    real_planes<P, R, INPLACE, G::ELEMS>(reinterpret_cast<double*>(s_in), p1);
+                    __syncthreads();
+#pragma unroll
+                    for (int rr = 0; rr < ROWS; ++rr)
+                        if (ract[rr]) fp64_row(warp * ROWS + rr, o[rr]);
+                    continue;
+                }
             }
 #pragma unroll
             for (int rr = 0; rr < ROWS; ++rr)
