@@ -7,6 +7,7 @@
 
 #include "prk_arith.cuh"
 #include "prk_internal.cuh"
+#include "prk_ptx.cuh"
 
 namespace prk {
 namespace {
@@ -110,6 +111,7 @@ __global__ void __launch_bounds__(ADD_THREADS) k_add(int64_t head, int64_t nvec,
     };
     T* in = static_cast<T*>(in_v);
     V* vec = reinterpret_cast<V*>(in + head);
+    chain_wait();
     const int64_t v0 = static_cast<int64_t>(blockIdx.x) * ADD_U * ADD_THREADS + threadIdx.x;
     V x[ADD_U];
 #pragma unroll
@@ -207,6 +209,7 @@ template <int DT>
 __global__ void __launch_bounds__(NORM_THREADS) k_norm_partial(int R, int64_t n, int64_t i_lo, int64_t i_hi,
                                                                const void* out_v, double* partial)
 {
+    chain_wait();
     double acc = 0.0;
     float ah = 0.0f, al = 0.0f;
     auto add_pair = [&](float h, float l) {
@@ -280,18 +283,11 @@ __global__ void __launch_bounds__(256) k_dadd_probe(double* sink, double step, i
 __global__ void __launch_bounds__(NORM_THREADS) k_norm_final(const double* partial, int count, double active,
                                                              double* result)
 {
+    chain_wait();
     double acc = 0.0;
     for (int k = threadIdx.x; k < count; k += NORM_THREADS) acc += partial[k];
     const double tot = block_sum<NORM_THREADS>(acc);
     if (threadIdx.x == 0) *result = tot / active;
-}
-
-int grid_for(int64_t work, int threads, int cap)
-{
-    int64_t b = (work + threads - 1) / threads;
-    if (b < 1) b = 1;
-    if (b > cap) b = cap;
-    return static_cast<int>(b);
 }
 
 }  // namespace
@@ -316,11 +312,7 @@ cudaError_t launch_add(int64_t n, int dtype, void* in, cudaStream_t s)
     // one block per ADD_U * ADD_THREADS vectors (2^31 - 1 of them would be 35 TB)
     const int64_t work = nvec > 0 ? (nvec + ADD_U - 1) / ADD_U : total;
     const unsigned blocks = static_cast<unsigned>(std::min<int64_t>((work + ADD_THREADS - 1) / ADD_THREADS, 0x7FFFFFFF));
-    if (dtype == FP64)
-        k_add<FP64><<<blocks, ADD_THREADS, 0, s>>>(head, nvec, total, in);
-    else
-        k_add<FP32C><<<blocks, ADD_THREADS, 0, s>>>(head, nvec, total, in);
-    return cudaGetLastError();
+    return launch_chained(dtype == FP64 ? k_add<FP64> : k_add<FP32C>, blocks, ADD_THREADS, 0, s, head, nvec, total, in);
 }
 
 cudaError_t launch_init(int64_t n, int dtype, void* in, void* out, cudaStream_t s)
@@ -345,15 +337,11 @@ cudaError_t launch_norm_rows(int R, int64_t n, int dtype, const void* out, int64
     const int64_t rows = i_hi > i_lo ? i_hi - i_lo : 0;
     const int blocks = static_cast<int>(rows < NORM_BLOCKS ? rows : NORM_BLOCKS);
     if (blocks > 0) {
-        if (dtype == FP64)
-            k_norm_partial<FP64><<<blocks, NORM_THREADS, 0, s>>>(R, n, i_lo, i_hi, out, partial);
-        else
-            k_norm_partial<FP32C><<<blocks, NORM_THREADS, 0, s>>>(R, n, i_lo, i_hi, out, partial);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        if (cudaError_t e = launch_chained(dtype == FP64 ? k_norm_partial<FP64> : k_norm_partial<FP32C>, blocks,
+                                           NORM_THREADS, 0, s, R, n, i_lo, i_hi, out, partial))
+            return e;
     }
-    k_norm_final<<<1, NORM_THREADS, 0, s>>>(partial, blocks, divisor, result_dev);
-    return cudaGetLastError();
+    return launch_chained(k_norm_final, 1, NORM_THREADS, 0, s, partial, blocks, divisor, result_dev);
 }
 
 cudaError_t launch_norm(int R, int64_t n, int dtype, const void* out, double* partial, double* result_dev, cudaStream_t s)

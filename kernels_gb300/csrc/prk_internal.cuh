@@ -8,6 +8,26 @@
 
 namespace prk {
 
+// Launch a kernel that begins with chain_wait (prk_ptx.cuh) so that its launch and its set-up overlap
+// the end of the stream's previous kernel. A run is launch after launch: star R=2, one application per
+// launch, us per application with plain launches and with these: n=200 6.28 and 3.52, n=1000 8.54 and
+// 6.69, n=2000 20.4 and 16.3, n=4096 82.3 and 79.1.
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A&&... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // One stencil application as the C ABI describes it (prk_gb300_stencil). The buffers hold the whole
 // n x n grid, or (nr > 0) a row slab of it: nr rows from grid row goff, row stride n
 // (prk_gb300_slab_run).

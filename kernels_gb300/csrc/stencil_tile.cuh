@@ -72,6 +72,7 @@ constexpr int FP32_MAX_STEPS = 65536;
 
 constexpr int SMEM_PER_SM = 228 * 1024;
 constexpr int SMEM_PER_CTA_MAX = 227 * 1024;
+constexpr int SMEM_DEFAULT_MAX = 48 * 1024;  // without cudaFuncAttributeMaxDynamicSharedMemorySize
 
 template <int DT, int R, int TH_ = 32>
 struct Geo {
@@ -2587,6 +2588,9 @@ __global__ void __launch_bounds__(THREADS, min_blocks<P, R, DT, STEPS, TH_>())
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
+    }
+    chain_wait();
+    if (threadIdx.x == 0) {
         mbar_arrive_expect_tx(bar, G::IN_BYTES + (has_out ? G::OUT_BYTES : 0));
         tma_load_2d(smem, &tm_in, static_cast<int32_t>(j0 - G::RA), static_cast<int32_t>(i0 - R), bar);
         if (has_out) tma_load_2d(smem + G::OUT_OFF, &tm_out, static_cast<int32_t>(j0), static_cast<int32_t>(i0), bar);
@@ -2610,8 +2614,9 @@ cudaError_t launch(const Launch& L)
     using C = Cfg<DT, TH_>;
     constexpr int SMEM = tile_smem<P, R, DT, TH_>();
     static_assert(SMEM <= SMEM_PER_CTA_MAX, "the tile and its tables must fit in shared memory");
-    if (cudaError_t e = cudaFuncSetAttribute(k_stencil_tile<P, R, DT, STEPS, TH_>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM))
-        return e;
+    if constexpr (SMEM > SMEM_DEFAULT_MAX)
+        if (cudaError_t e = cudaFuncSetAttribute(k_stencil_tile<P, R, DT, STEPS, TH_>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM))
+            return e;
     const int64_t nr = L.nr > 0 ? L.nr : L.n;
     if (L.row0 < 0 || L.row0 >= nr || L.rows < 0 || (STEPS == 0 && L.depth < 1) || L.goff < 0 || L.goff + nr > L.n)
         return cudaErrorInvalidValue;
@@ -2619,10 +2624,8 @@ cudaError_t launch(const Launch& L)
     const int64_t tx = (L.n + C::TW - 1) / C::TW, ty = (rows + C::TH - 1) / C::TH;
     if (ty > 65535) return cudaErrorInvalidValue;
     const dim3 grid(static_cast<unsigned>(tx), static_cast<unsigned>(ty));
-    k_stencil_tile<P, R, DT, STEPS, TH_><<<grid, THREADS, SMEM, L.stream>>>(L.tm_in, L.tm_out, L.n, L.in_next, L.out,
-                                                                             L.status, L.depth, L.row0, L.goff,
-                                                                             L.row0 + rows);
-    return cudaGetLastError();
+    return launch_chained(k_stencil_tile<P, R, DT, STEPS, TH_>, grid, THREADS, SMEM, L.stream, L.tm_in, L.tm_out, L.n,
+                          L.in_next, L.out, L.status, L.depth, L.row0, L.goff, L.row0 + rows);
 }
 
 // Supported temporal depths; a run of any length is split into launches of these, or runs in one

@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(tile::THREADS, plain_min_blocks<P, R, DT, STEP
     const int64_t i0 = row0 + static_cast<int64_t>(blockIdx.y) * C::TH;
     const int64_t j0 = static_cast<int64_t>(blockIdx.x) * C::TW;
     const bool has_out = tile::tile_has_out(i0 + goff, j0, n, R, C::TW, C::TH);
+    chain_wait();
     if constexpr (S::TBL) {
         stage_async<R, DT>(smem, in, out, n, nr, i0, j0, has_out);
         tile::process_tile<P, R, DT, STEPS, tile::OUT_SMEM>(smem, s_red, i0, j0, n, has_out, in_next, out, false,
@@ -153,8 +154,9 @@ cudaError_t launch(const Args& a)
 {
     using C = tile::Cfg<DT>;
     constexpr int SM = Smem<P, DT, R>::BYTES;
-    if (cudaError_t e = cudaFuncSetAttribute(k_stencil_plain<P, R, DT, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM))
-        return e;
+    if constexpr (SM > tile::SMEM_DEFAULT_MAX)
+        if (cudaError_t e = cudaFuncSetAttribute(k_stencil_plain<P, R, DT, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM))
+            return e;
     const int64_t nr = a.nr > 0 ? a.nr : a.n;
     if (a.row0 < 0 || a.row0 >= nr || a.rows < 0 || a.depth < 1 || a.goff < 0 || a.goff + nr > a.n)
         return cudaErrorInvalidValue;
@@ -162,9 +164,8 @@ cudaError_t launch(const Args& a)
     const int64_t tx = (a.n + C::TW - 1) / C::TW, ty = (rows + C::TH - 1) / C::TH;
     if (ty > 65535) return cudaErrorInvalidValue;
     const dim3 grid(static_cast<unsigned>(tx), static_cast<unsigned>(ty));
-    k_stencil_plain<P, R, DT, STEPS><<<grid, tile::THREADS, SM, a.stream>>>(a.in, a.in_next, a.out, a.n, a.depth, a.row0,
-                                                                          nr, a.goff, a.row0 + rows);
-    return cudaGetLastError();
+    return launch_chained(k_stencil_plain<P, R, DT, STEPS>, grid, tile::THREADS, SM, a.stream, a.in, a.in_next, a.out,
+                          a.n, a.depth, a.row0, nr, a.goff, a.row0 + rows);
 }
 
 // One application (depth 1: the STEPS = 1 kernel), `depth` applications in one launch (STEPS = 0), or
