@@ -468,9 +468,10 @@ struct IntCheck {
 };
 
 // S[rr][k] += M * S of the thread's CPT points of ROWS consecutive rows; u points at (r0, c0) of the tile.
-// Row by row of the tile: each row segment is read once and enters every output row it is a tap of.
+// Row by row of the tile: each row segment is read once and enters every output row it is a tap of. own
+// (when given) gets the values of the thread's points.
 template <int P, int R, int CPT, int ROWS, int RA>
-__device__ __forceinline__ void int_rows(const float* u, int ld, float (&S)[ROWS][CPT])
+__device__ __forceinline__ void int_rows(const float* u, int ld, float (&S)[ROWS][CPT], float (*own)[CPT] = nullptr)
 {
     constexpr IntCoefs<P, R> C = make_int_coefs<P, R>();
 #pragma unroll
@@ -494,6 +495,10 @@ __device__ __forceinline__ void int_rows(const float* u, int ld, float (&S)[ROWS
         if (P == GRID || (q >= 0 && q < ROWS)) {
             float seg[CPT + 2 * RA];
             ld_seg<CPT + 2 * RA>(u + q * ld - RA, seg);
+            if (own && q >= 0 && q < ROWS) {
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) own[q][k] = seg[k + RA];
+            }
             taps(std::integral_constant<int, RA>{}, seg);
         } else {  // star: a row above or below the thread's is a vertical tap only
             float seg[CPT];
@@ -504,14 +509,16 @@ __device__ __forceinline__ void int_rows(const float* u, int ld, float (&S)[ROWS
 }
 
 // (o_hi, o_lo) += (t + tl) / M, renormalised, for whole t and tl (t a float's 24 bits, |tl| far smaller):
-// q near t / M, the remainder t - q M exact (a small multiple of q's last bit), and the remainder's share
-// of the quotient as the low word. Exact where M divides t, as it does for a PRK field.
+// q = t / M rounded (one correction of t * (1 / M)), the remainder t - q M exact (a small multiple of q's
+// last bit), and the remainder's share of the quotient as the low word. Exact where M divides t, as it
+// does for a PRK field; within 2^-46.9 of the quotient otherwise.
 template <int P, int R>
 __device__ __forceinline__ void int_add(uint64_t& o, float t, float tl)
 {
     constexpr int M = common_den<P, R>();
     constexpr float INV = static_cast<float>(1.0 / M);
-    const float q = __fmul_rn(t, INV);
+    const float q0 = __fmul_rn(t, INV);
+    const float q = __fmaf_rn(__fmaf_rn(-q0, static_cast<float>(M), t), INV, q0);
     const float rem = __fmaf_rn(-q, static_cast<float>(M), t);
     float oh = __uint_as_float(static_cast<uint32_t>(o)), ol = __uint_as_float(static_cast<uint32_t>(o >> 32));
     df_add(oh, ol, q, __fmul_rn(__fadd_rn(rem, tl), INV));
@@ -2327,16 +2334,15 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             if (inted) {
                 // The integer route: M * S of every application summed exactly, out read and updated once
                 // at the end. `sums` applications fit the FP32 sum; it then goes to an integer.
+                // The in += 1 of the thread's own points from the values its sums have just read, the halo beside
+                // them; a pass over the whole tile where the extra registers cost more (n=8192, whole runs,
+                // us per application: star R=1 47 to 43, R=2 51 to 48; launches of eight, R=5 85 to 88).
+                constexpr bool FUSED_ADVANCE = P == STAR && R <= 2;
                 float a[ROWS][CPT] = {};
                 int acc[ROWS][CPT] = {};
                 int held = 0;
 #pragma unroll 1
                 for (int t = 0; t < nsteps; ++t) {
-                    if (t > 0) {
-                        __syncthreads();
-                        advance_f32<G::ELEMS>(s_in);
-                        __syncthreads();
-                    }
                     if (held == sums) {
                         held = 0;
 #pragma unroll
@@ -2348,8 +2354,24 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                             }
                     }
                     ++held;
-                    if (has_out)
-                        int_rows<P, R, CPT, ROWS, G::RA>(s_in + (warp * ROWS + R) * G::SW + G::RA + c0, G::SW, a);
+                    float* const mine = s_in + (warp * ROWS + R) * G::SW + G::RA + c0;
+                    float own[ROWS][CPT];
+                    if (has_out) int_rows<P, R, CPT, ROWS, G::RA>(mine, G::SW, a, FUSED_ADVANCE ? own : nullptr);
+                    if (t + 1 < nsteps) {  // in += 1
+                        __syncthreads();
+                        if (FUSED_ADVANCE && has_out) {
+#pragma unroll
+                            for (int rr = 0; rr < ROWS; ++rr) {
+#pragma unroll
+                                for (int k = 0; k < CPT; ++k) own[rr][k] = __fadd_rn(own[rr][k], 1.0f);
+                                st_vec(mine + rr * G::SW, own[rr]);
+                            }
+                            advance_halo_f32<G::SW, G::SH, R, G::RA>(s_in, s_in);
+                        } else {
+                            advance_f32<G::ELEMS>(s_in);
+                        }
+                        __syncthreads();
+                    }
                 }
 #pragma unroll
                 for (int rr = 0; rr < ROWS; ++rr) {
