@@ -355,7 +355,7 @@ def run_gb300(args) -> None:
                                                 "peak_source": "prk_gb300_probe_dadd, measured in this run"},
                               "fixed_point_adds": {"adds_per_point": fixed_adds,
                                                    "achieved_adds_per_s": round(fixed_adds * pts / per_g, 1),
-                                                   "where": "integer pipes, about 25 integer instructions each"},
+                                                   "where": "integer pipes, about 10 instructions each with their two table reads"},
                               "note": "the weights are not powers of two, so every product and every partial sum "
                                       "of the reference's chain is rounded: each of the chain's adds runs either "
                                       "as a binary64 add or as its exact fixed-point image"}}

@@ -17,13 +17,13 @@ BATCH_SEED = 20260101
 
 # Measured time per point and application of each stencil on one GB300, as PRK GFLOP/s of tuned
 # runs at n = 32768 (kernels_gb300.configs sweep): the cost model of the split below. The FP64
-# stencils with power-of-two weights take the exact integer routes and run an order of magnitude
+# stencils with power-of-two weights take the exact integer routes and run several times
 # faster than the ones whose every add is rounded; FP32C is fast for all of them.
 SWEEP_GFLOPS = {
-    "fp64": {(0, 1): 18116, (0, 2): 27871, (0, 3): 1930, (0, 4): 2061, (0, 5): 2027,
-             (1, 1): 28738, (1, 2): 2439, (1, 3): 2394, (1, 4): 2237, (1, 5): 2175},
-    "fp32c": {(0, 1): 13915, (0, 2): 16571, (0, 3): 17538, (0, 4): 17514, (0, 5): 17170,
-              (1, 1): 17556, (1, 2): 22891, (1, 3): 27141, (1, 4): 33038, (1, 5): 33318},
+    "fp64": {(0, 1): 18097, (0, 2): 27835, (0, 3): 4417, (0, 4): 4684, (0, 5): 4658,
+             (1, 1): 28707, (1, 2): 5769, (1, 3): 6026, (1, 4): 6008, (1, 5): 5980},
+    "fp32c": {(0, 1): 19905, (0, 2): 30623, (0, 3): 35544, (0, 4): 42358, (0, 5): 39518,
+              (1, 1): 28174, (1, 2): 57295, (1, 3): 72564, (1, 4): 77203, (1, 5): 77237},
 }
 
 
