@@ -151,13 +151,13 @@ __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const v
         if (i0 >= R && j0 >= G::RA && i0 - R + G::SH <= nr && j0 - G::RA + G::SW <= n) {  // every element loaded
             store([&](int q) {
                 const float u = __fsub_rn(v[q], it.ref);
-                if ((q + 1) * tile::THREADS <= G::ELEMS || threadIdx.x + q * tile::THREADS < G::ELEMS) check.add(u);
+                if ((q + 1) * tile::THREADS <= G::ELEMS || threadIdx.x + q * tile::THREADS < G::ELEMS) check.add(v[q], u);
                 return u;
             });
         } else {
             store([&](int q) {
                 const float u = __fsub_rn(v[q], it.ref);
-                if (loaded >> q & 1u) check.add(u);
+                if (loaded >> q & 1u) check.add(v[q], u);
                 return u;
             });
         }

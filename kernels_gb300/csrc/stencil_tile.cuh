@@ -443,13 +443,14 @@ struct IntTile {
 // |x| < 2^22 and whole.
 __device__ __forceinline__ bool whole_f32(float x) { return __fsub_rn(__fadd_rn(x, 12582912.0f), 12582912.0f) == x; }
 
-// The tile's values u = in - ref: whole, and the largest |u|. in is then whole, as ref is.
+// The tile's values: in whole, and the largest |u|, u = in - ref. Asked of in, not of u: the difference of
+// a small value and a whole ref rounds to a whole number. With ref whole and in below 2^22, u is exact.
 struct IntCheck {
     bool whole = true;
     float most = 0.0f;
-    __device__ __forceinline__ void add(float u)
+    __device__ __forceinline__ void add(float v, float u)
     {
-        whole = whole && whole_f32(u);
+        whole = whole && whole_f32(v);
         most = fmaxf(most, fabsf(u));
     }
     // The block's verdict (a barrier, or two where the values are not near): IntTile::sums.
@@ -458,7 +459,9 @@ struct IntCheck {
     {
         using Near = IntBound<P, R, INT_NEAR>;
         using Wide = IntBound<P, R, int_wide<P, R>()>;
-        const bool ok = whole && fabsf(ref) < 8388608.0f && rintf(ref) == ref;  // in + steps below 2^24
+        // |in| < |ref| + 2^17 <= 2^22 where |u| < B, as whole_f32 needs; in + steps stays below 2^24
+        static_assert(int_wide<P, R>() <= (1 << 17), "in below 2^22");
+        const bool ok = whole && fabsf(ref) <= 4194304.0f - 131072.0f && rintf(ref) == ref;
         if (__syncthreads_and(ok && most < static_cast<float>(INT_NEAR) && nsteps <= Near::STEPS)) return Near::SUMS;
         if (int_wide<P, R>() > INT_NEAR &&
             __syncthreads_and(ok && most < static_cast<float>(int_wide<P, R>()) && nsteps <= Wide::STEPS))
@@ -2021,8 +2024,9 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                 float* e = reinterpret_cast<float*>(&u[q]);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    e[k] = __fsub_rn(e[k], uref);
-                    if (!edge || inside(4 * v + k)) check.add(e[k]);
+                    const float x = e[k];
+                    e[k] = __fsub_rn(x, uref);
+                    if (!edge || inside(4 * v + k)) check.add(x, e[k]);
                 }
             }
             sums = check.sums<P, R>(uref, nsteps);

@@ -121,3 +121,33 @@ def test_more_applications_than_one_sum_takes(cuda, pattern, r):
             inner = (slice(r, n - r), slice(r, n - r))
             assert (np.abs(got[..., 0][inner].astype(np.longdouble) + got[..., 1][inner] - s) <= 1e-6 * m).all()
         assert np.array_equal(in_b.cpu().numpy(), a + np.float32(apps))
+
+
+@pytest.mark.parametrize("pattern,r", ALL)
+@pytest.mark.parametrize("n", [180, 149])
+@pytest.mark.parametrize("base", [64, -100000])
+def test_small_value_among_whole_ones(cuda, pattern, r, n, base):
+    """A value of 2^-20 whose difference from the tile's middle rounds to a whole number: the tile keeps the
+    group sums, in += 1 keeps the value (its sums with 1..6 are exact in FP32), and the points around it,
+    in a block of zeros, get its taps."""
+    a = np.full((n, n), base, np.float32)
+    a[4:28, 8:32] = 0.0
+    a[16, 20] = 2.0 ** -20
+    zeros, apps = np.zeros((n, n), np.float32), 6
+
+    def fresh():
+        return cuda.from_numpy(a.copy()).cuda(), cuda.zeros((n, n, 2), device="cuda")
+
+    in_a, out = fresh()
+    res = kg.run(pattern, r, apps - 1, in_a, cuda.empty_like(in_a), out, whole=True)
+    check(pattern, r, a, zeros, out.cpu().numpy(), apps, whole=False)
+    assert np.array_equal(res.final_in.cpu().numpy().astype(np.float64), a.astype(np.float64) + apps)
+    in_a, out = fresh()
+    kg.Batch([(pattern, r, in_a, cuda.empty_like(in_a), out)], whole=True).run(apps - 1)
+    check(pattern, r, a, zeros, out.cpu().numpy(), apps, whole=False)
+    for nxt in (False, True):
+        in_, out = fresh()
+        nx = cuda.empty_like(in_) if nxt else None
+        kg.apply(pattern, r, in_, out, nx)
+        check(pattern, r, a, zeros, out.cpu().numpy(), 1, whole=False)
+        assert nx is None or np.array_equal(nx.cpu().numpy().astype(np.float64), a.astype(np.float64) + 1)
