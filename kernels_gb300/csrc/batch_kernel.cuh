@@ -106,7 +106,7 @@ __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const v
     using T = typename tile::Cfg<DT>::T;
     constexpr int PER = (G::ELEMS + tile::THREADS - 1) / tile::THREADS;
     constexpr int DR = tile::THREADS / G::SW, DC = tile::THREADS % G::SW;
-    const T* __restrict__ in = static_cast<const T*>(in_v);
+    const T* in = static_cast<const T*>(in_v);
     T* s_in = reinterpret_cast<T*>(smem);
     const uint32_t un = static_cast<uint32_t>(n), unr = static_cast<uint32_t>(nr);  // n, nr <= NMAX < 2^31
     int r = threadIdx.x / G::SW, c = threadIdx.x - (threadIdx.x / G::SW) * G::SW;

@@ -11,7 +11,10 @@ namespace prk {
 
 // Programmatic dependent launch: a kernel launched with launch_chained (prk_internal.cuh) may start while
 // the stream's previous kernel still runs. chain_wait returns once that kernel has completed and its
-// writes are visible; nothing before it may touch global memory. The previous kernel gives no early
+// writes are visible; nothing before it may touch global memory. That kernel still writes the next one's
+// buffers while the next one runs, so a chained kernel's pointers carry no __restrict__: a load through a
+// const __restrict__ parameter is one of memory that no one writes while the kernel runs, and a compiler may
+// move it above the wait. The previous kernel gives no early
 // signal (griddepcontrol.launch_dependents): blocks that wait for it in its last wave's free slots spread
 // the next grid unevenly over the SMs (star R=2, us per application, without a signal, with one at the
 // kernel's end and at its start: n=1000 6.69, 8.58, 8.89; n=4096 79.1, 81.3, 81.5).

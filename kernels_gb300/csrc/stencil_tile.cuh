@@ -1787,7 +1787,7 @@ __device__ __forceinline__ bool tile_has_out(int64_t i0, int64_t j0, int64_t n, 
 // Rows from row_end on (in the arrays) are not stored; the interior test uses grid rows.
 template <int P, int R, int DT, int STEPS, int OUT_SRC = OUT_SMEM, int TH_ = 32>
 __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, int64_t i0, int64_t j0, int64_t n,
-                                             bool has_out, void* __restrict__ in_next_v, void* __restrict__ out_v,
+                                             bool has_out, void* in_next_v, void* out_v,
                                              bool vec_ok, int depth, int64_t goff, int64_t row_end,
                                              unsigned char* tbl, const IntTile& pre = IntTile{})
 {
@@ -2599,7 +2599,7 @@ constexpr int min_blocks()
 template <int P, int R, int DT, int STEPS, int TH_>
 __global__ void __launch_bounds__(THREADS, min_blocks<P, R, DT, STEPS, TH_>())
     k_stencil_tile(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out,
-                   const int64_t n, void* __restrict__ in_next_v, void* __restrict__ out_v, unsigned* __restrict__ status,
+                   const int64_t n, void* in_next_v, void* out_v, unsigned* status,
                    const int depth, const int64_t row0, const int64_t goff, const int64_t row_end)
 {
     using G = Geo<DT, R, TH_>;

@@ -56,7 +56,7 @@ __device__ __forceinline__ void stage_async(unsigned char* smem, const void* in_
     constexpr int E = static_cast<int>(sizeof(T));
     constexpr int PER = (G::ELEMS + tile::THREADS - 1) / tile::THREADS;
     constexpr int DR = tile::THREADS / G::SW, DC = tile::THREADS % G::SW;
-    const T* __restrict__ in = static_cast<const T*>(in_v);
+    const T* in = static_cast<const T*>(in_v);
     T* s_in = reinterpret_cast<T*>(smem);
     const uint32_t un = static_cast<uint32_t>(n), unr = static_cast<uint32_t>(nr);  // n, nr <= NMAX < 2^31
     int c = threadIdx.x - (threadIdx.x / G::SW) * G::SW;
@@ -82,7 +82,7 @@ __device__ __forceinline__ void stage_async(unsigned char* smem, const void* in_
     }
     if (has_out) {
         static_assert((C::TW & (C::TW - 1)) == 0 && (C::TW * C::TH) % tile::THREADS == 0, "out tile layout");
-        const uint64_t* __restrict__ out = static_cast<const uint64_t*>(out_v);
+        const uint64_t* out = static_cast<const uint64_t*>(out_v);
         uint64_t* o_tile = reinterpret_cast<uint64_t*>(smem + G::OUT_OFF);
 #pragma unroll
         for (int q = 0; q < C::TW * C::TH / tile::THREADS; ++q) {
@@ -109,8 +109,8 @@ __device__ __forceinline__ void stage_async(unsigned char* smem, const void* in_
 // L1).
 template <int P, int R, int DT, int STEPS>
 __global__ void __launch_bounds__(tile::THREADS, plain_min_blocks<P, R, DT, STEPS>())
-    k_stencil_plain(const void* __restrict__ in, void* __restrict__ in_next, void* __restrict__ out, const int64_t n,
-                    const int depth, const int64_t row0, const int64_t nr, const int64_t goff, const int64_t row_end)
+    k_stencil_plain(const void* in, void* in_next, void* out, const int64_t n, const int depth, const int64_t row0,
+                    const int64_t nr, const int64_t goff, const int64_t row_end)
 {
     using C = tile::Cfg<DT>;
     using S = Smem<P, DT, R>;
