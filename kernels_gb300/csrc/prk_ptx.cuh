@@ -30,6 +30,12 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
 
+// End the barrier's life: its memory may then hold something else. Every thread has left its waits.
+__device__ __forceinline__ void mbar_inval(uint64_t* bar)
+{
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
 // Make the initialised barrier visible to the async (TMA) proxy.
 __device__ __forceinline__ void fence_mbar_init()
 {

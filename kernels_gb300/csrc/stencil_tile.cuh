@@ -1444,7 +1444,8 @@ __device__ __forceinline__ void table_chain(const int32_t* sp, const unsigned ch
 //  - fl(v / (2^k d)) = 2^-k fl(v / d), so the weights whose denominators share their odd part share one
 //    rounded product per value, and every tap that uses it is again a fused multiply-add by +-2^-k. The
 //    products of a family of weights are computed once per value into a plane of the tile in shared
-//    memory (of `out` words and tables that this path does not need by then) instead of once per tap.
+//    memory (over the `out` words, the TMA kernel's barrier, which has ended, and the tables: this path
+//    needs none of them by then) instead of once per tap.
 // A family that has no plane multiplies per tap. Binary64 instructions per point, before and now: star
 // R=2 17 and 10, star R=3 24 and 16, grid R=2 37 and 23. At n=8192, one fused application, us: star R=2
 // 2185 to 1293, R=3 3199 to 2019, R=4 4215 to 2493, R=5 5229 to 3907; grid R=2 4850 to 2974, R=3 9926 to
@@ -2047,7 +2048,9 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
     constexpr bool INPLACE = one_application(STEPS) && two_families<P, R>();
     constexpr bool PLANES = DT == FP64 && !EXACT;  // the power-of-two stencils need no plane beside the tile
     bool real = false;
-    double* p1 = nullptr;  // plane 1: over the out words (read into registers first) and the tables
+    // plane 1: from the out words on (read into registers first), over the reduction words, the TMA kernel's
+    // barrier (ended by then) and the tables
+    double* p1 = nullptr;
     if constexpr (DT == FP64) {
         if ((EXACT ? one_application(STEPS) && !fexact && unit == fx::NOT_FIXED : !iwhole) && (!PLANES || tbl)) {
             bool ok = true;
@@ -2629,6 +2632,8 @@ __global__ void __launch_bounds__(THREADS, min_blocks<P, R, DT, STEPS, TH_>())
         mbar_wait_bounded(bar, 0);  // let the copies land before the CTA's shared memory is released
         return;
     }
+    // process_tile may put a plane of products over the barrier, several block barriers further on
+    if (table_route<P, R, DT>() && threadIdx.x == 0) mbar_inval(bar);
     process_tile<P, R, DT, STEPS, OUT_SMEM, TH_>(smem, s_red, i0, j0, n, has_out, in_next_v, out_v, true, depth, goff,
                                                  row_end,
                                                  table_route<P, R, DT>() ? smem + table_offset<DT, R, TH_>() : nullptr);
