@@ -180,8 +180,9 @@ int prk_gb300_norm_noalloc(int radius, int64_t n, int dtype, const void* out, do
 int prk_gb300_config(int key, int value);
 
 /* Reads and clears the device status word of the current device: PRK_OK, or PRK_ERR_TIMEOUT when a
- * kernel's bounded wait on its tile loads gave up since the last check. Synchronises the device.
- * prk_gb300_run checks it after every run. */
+ * kernel's bounded wait on its tile loads gave up since the last check. Waits for what the legacy
+ * default stream waits for; wait for work on non-blocking streams first. Runs, batch runs and host-buffer
+ * runs check it after their own work. */
 int prk_gb300_status(void);
 
 /* ---- Autotuner ----------------------------------------------------------------------------

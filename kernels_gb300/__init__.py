@@ -85,7 +85,8 @@ def set_kernel(choice: int) -> int:
 
 
 def status() -> None:
-    """Raise if a kernel's bounded wait gave up since the last check (synchronises the device)."""
+    """Raise if a kernel's bounded wait gave up since the last check. Waits for the default stream;
+    wait for work on other streams first."""
     check(load().prk_gb300_status())
 
 

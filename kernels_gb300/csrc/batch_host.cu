@@ -294,7 +294,7 @@ int prk_gb300_batch_run(prk_gb300_batch* b, int iterations, int flags, double* e
         if (elapsed_s) *elapsed_s = ms * 1e-3;
         for (size_t gi = 0; gi < b->groups.size(); ++gi)
             for (int k : b->groups[gi].members) b->final_in[k] = parity[gi];
-        rc = prk_gb300_status();
+        rc = prk::read_status();
     } while (false);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);

@@ -212,8 +212,9 @@ int launch_steps(int pattern, int radius, int64_t n, int dtype, int steps, const
     return PRK_OK;
 }
 
-// Reads and clears the device status word. The caller has waited for the kernels it asks about.
-int read_status()
+}  // namespace
+
+int prk::read_status()
 {
     DevScratch d;
     if (int rc = dev_scratch(&d)) return rc;
@@ -225,11 +226,17 @@ int read_status()
     return PRK_OK;
 }
 
-// The same, after everything on the device.
+namespace {
+
+// The same, after what the legacy stream waits for. Not after everything on the device: while another
+// stream is being captured, cudaDeviceSynchronize fails and invalidates that capture.
 int check_status()
 {
-    PRK_CUDA(cudaDeviceSynchronize(), "status synchronize");
-    return read_status();
+    DevScratch d;
+    if (int rc = dev_scratch(&d)) return rc;
+    double word = 0.0;  // a copy on the legacy stream, for its wait alone
+    PRK_CUDA(cudaMemcpy(&word, d.norm, sizeof word, cudaMemcpyDeviceToHost), "status wait");
+    return prk::read_status();
 }
 
 }  // namespace
@@ -504,7 +511,7 @@ int prk_gb300_run(int pattern, int radius, int64_t n, int dtype, int iterations,
         cudaEventElapsedTime(&ms, e0, e1);
         if (elapsed_s) *elapsed_s = ms * 1e-3;
         if (final_in) *final_in = unfused ? 0 : cur;
-        rc = read_status();
+        rc = prk::read_status();
     } while (false);
     if (ge) cudaGraphExecDestroy(ge);
     if (g) cudaGraphDestroy(g);
@@ -661,7 +668,7 @@ int run_host_banded(HostWorkspace& ws, int pattern, int radius, int64_t n, int d
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, span.ev[0], span.ev[1]);
     if (kernel_s) *kernel_s = ms * 1e-3;
-    return check_status();
+    return prk::read_status();
 }
 
 }  // namespace

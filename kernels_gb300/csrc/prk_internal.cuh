@@ -106,4 +106,7 @@ int table_route_split(int pattern, int R, int depth, int* fixed_adds, int* binar
 // Records `msg` as the calling thread's prk_gb300_last_error() and returns `code` (capi.cu).
 int record_error(int code, const char* msg);
 
+// Reads and clears the current device's status word. The caller has waited for the kernels it asks about.
+int read_status();
+
 }  // namespace prk
