@@ -25,7 +25,9 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t 
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();  // reported here; a later launch's check is not to find it again
+    return e;
 }
 
 // One stencil application as the C ABI describes it (prk_gb300_stencil). The buffers hold the whole
