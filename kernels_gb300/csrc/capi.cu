@@ -9,6 +9,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/prk_gb300.h"
@@ -65,23 +66,22 @@ bool overlaps(const void* a, int64_t abytes, const void* b, int64_t bbytes)
     return pa < pb + bbytes && pb < pa + abytes;
 }
 
-// Library-owned scratch: NORM_BLOCKS partial sums for the norm in device memory; in pinned host memory
-// that the kernels write, the status word the tile kernels set when a bounded wait gives up and
-// NORM_RESULTS slots for norms. A run and a norm then read their verdict and value after the wait they
-// make anyway instead of through a blocking copy each (star R=2, n=200, ten iterations: 82 to 70 us, its
+// Library-owned scratch: in device memory, NORM_BLOCKS partial sums for each of NORM_SLOTS norms at a
+// time (512 KB); in pinned host memory that the kernels write, the status word the tile kernels set when
+// a bounded wait gives up and the norms' results. A run and a norm then read their verdict and value
+// after the wait they make anyway instead of through a blocking copy each (star R=2, n=200, ten iterations: 82 to 70 us, its
 // norm 28 to 22 us). One allocation per device, kept until the process exits, with the id of the context
 // it was made in: in a new context on the device (after cudaDeviceReset, which freed it) it is allocated
 // again.
-constexpr int NORM_RESULTS = 64;
+constexpr int NORM_SLOTS = 64;
 struct DevScratch {
-    double* norm = nullptr;
+    double* norm = nullptr;  // NORM_SLOTS * NORM_BLOCKS partial sums
     volatile unsigned* status_host = nullptr;  // the status word, and its address on the device
     unsigned* status = nullptr;
-    volatile double* result_host = nullptr;    // NORM_RESULTS results, and their address on the device
+    volatile double* result_host = nullptr;    // NORM_SLOTS results, and their address on the device
     double* result = nullptr;
     unsigned long long context = 0;
 };
-std::atomic<unsigned> g_norm_slot{0};
 std::mutex g_scratch_mu;
 std::vector<DevScratch> g_scratch;
 
@@ -108,8 +108,8 @@ int dev_scratch(DevScratch* out)
         // capture.
         RelaxedCapture relaxed;
         void* p = nullptr;
-        const size_t bytes = (prk::NORM_BLOCKS + 1) * sizeof(double);
-        constexpr size_t HOST_BYTES = 256 + NORM_RESULTS * sizeof(double);
+        constexpr size_t bytes = static_cast<size_t>(NORM_SLOTS) * prk::NORM_BLOCKS * sizeof(double);
+        constexpr size_t HOST_BYTES = 256 + NORM_SLOTS * sizeof(double);
         cudaError_t e = cudaMalloc(&p, bytes);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -141,16 +141,53 @@ int dev_scratch(DevScratch* out)
     return PRK_OK;
 }
 
+// A norm's place in the scratch, held while it lives: norms of several threads, on streams of their own,
+// run at the same time. With every place taken it waits for a norm to end.
+class NormSlot {
+public:
+    NormSlot()
+    {
+        uint64_t used = taken_.load(std::memory_order_relaxed);
+        for (;;) {
+            if (used == ~0ull) {
+                std::this_thread::yield();
+                used = taken_.load(std::memory_order_relaxed);
+                continue;
+            }
+            const uint64_t bit = ~used & (used + 1);  // the lowest free place
+            if (taken_.compare_exchange_weak(used, used | bit, std::memory_order_acquire, std::memory_order_relaxed)) {
+                bit_ = bit;
+                while (bit >> index > 1) ++index;
+                return;
+            }
+        }
+    }
+    ~NormSlot() { taken_.fetch_and(~bit_, std::memory_order_release); }
+    NormSlot(const NormSlot&) = delete;
+    NormSlot& operator=(const NormSlot&) = delete;
+    int index = 0;
+
+private:
+    static_assert(NORM_SLOTS == 64, "a bit per place");
+    static std::atomic<uint64_t> taken_;
+    uint64_t bit_ = 0;
+};
+std::atomic<uint64_t> NormSlot::taken_{0};
+
 // A norm over array rows [i_lo, i_hi) on stream s, waited for.
 int norm_rows(int radius, int64_t n, int dtype, const void* out, int64_t i_lo, int64_t i_hi, double divisor, double* value,
               cudaStream_t s)
 {
     DevScratch d;
     if (int rc = dev_scratch(&d)) return rc;
-    const unsigned slot = g_norm_slot.fetch_add(1, std::memory_order_relaxed) % NORM_RESULTS;
-    PRK_CUDA(prk::launch_norm_rows(radius, n, dtype, out, i_lo, i_hi, divisor, d.norm, d.result + slot, s), "norm launch");
-    PRK_CUDA(cudaStreamSynchronize(s), "norm synchronize");
-    *value = d.result_host[slot];
+    const NormSlot slot;
+    const cudaError_t launched = prk::launch_norm_rows(radius, n, dtype, out, i_lo, i_hi, divisor,
+                                                       d.norm + static_cast<int64_t>(slot.index) * prk::NORM_BLOCKS,
+                                                       d.result + slot.index, s);
+    const cudaError_t waited = cudaStreamSynchronize(s);  // also for a first kernel whose second was refused
+    PRK_CUDA(launched, "norm launch");
+    PRK_CUDA(waited, "norm synchronize");
+    *value = d.result_host[slot.index];
     return PRK_OK;
 }
 
