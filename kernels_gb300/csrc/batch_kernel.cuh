@@ -94,10 +94,10 @@ struct Layout {
 // outside the arrays (nr rows of n columns), all loads issued before the first shared-memory store.
 // Thread t takes elements t, t + THREADS, ... of the row-major tile; its row, column and grid offset
 // advance by constants from one element to the next (one division per thread, none per element).
-// FP32C: the values are checked for the integer route (tile::IntTile) on their way from the registers
-// and stored as that route wants them, or as they are when some value fails; the barrier that ends the
-// staging collects the verdict, so the check adds no pass over the tile and no barrier. row_hi: the first
-// array row no point reads.
+// FP32C: the values are checked for the integer route (tile::IntTile) in their registers and stored as the
+// tile's route wants them. The tile's middle and first values are asked first, by every thread: a field of
+// real numbers then pays for two loads, not for the check and a vote. row_hi: the first array row no point
+// reads.
 template <int P, int R, int DT, int STEPS>
 __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const void* in_v, int64_t n, int64_t nr,
                                                     int64_t i0, int64_t j0, int64_t row_hi, int nsteps)
@@ -109,36 +109,38 @@ __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const v
     const T* in = static_cast<const T*>(in_v);
     T* s_in = reinterpret_cast<T*>(smem);
     const uint32_t un = static_cast<uint32_t>(n), unr = static_cast<uint32_t>(nr);  // n, nr <= NMAX < 2^31
-    int r = threadIdx.x / G::SW, c = threadIdx.x - (threadIdx.x / G::SW) * G::SW;
-    int gi = static_cast<int>(i0) - R + r, gj = static_cast<int>(j0) - G::RA + c;
-    int64_t off = static_cast<int64_t>(gi) * n + gj;
+    // every element of the thread in turn: f(q, whether it lies in the arrays, its offset)
+    auto walk = [&](auto f) {
+        int r = threadIdx.x / G::SW, c = threadIdx.x - (threadIdx.x / G::SW) * G::SW;
+        int gi = static_cast<int>(i0) - R + r, gj = static_cast<int>(j0) - G::RA + c;
+        int64_t off = static_cast<int64_t>(gi) * n + gj;
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int idx = threadIdx.x + q * tile::THREADS;
+            f(q, ((q + 1) * tile::THREADS <= G::ELEMS || idx < G::ELEMS) && static_cast<uint32_t>(gi) < unr &&
+                     static_cast<uint32_t>(gj) < un, off);
+            c += DC;
+            gi += DR;
+            gj += DC;
+            off += DR * n + DC;
+            if (c >= G::SW) {
+                c -= G::SW;
+                gi += 1;
+                gj -= G::SW;
+                off += n - G::SW;
+            }
+        }
+    };
     tile::IntTile it;
     constexpr bool CHECK = tile::int_route<P, R, DT, STEPS, true>();
-    if constexpr (CHECK) {  // the value nearest the tile's middle inside the grid
+    float corner = 0.0f;
+    if constexpr (CHECK) {  // the value nearest the tile's middle inside the grid, and the tile's first
         const int64_t rm = min(i0 - R + G::SH / 2, row_hi - 1), cm = min(j0 - G::RA + G::SW / 2, n - 1);
         it.ref = in[rm * n + cm];
+        corner = in[i0 * n + j0];
     }
     T v[PER];
-    uint32_t loaded = 0;
-    static_assert(PER <= 32, "one bit per element of a thread");
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {  // all loads first, then the shared-memory stores
-        const int idx = threadIdx.x + q * tile::THREADS;
-        const bool ok = ((q + 1) * tile::THREADS <= G::ELEMS || idx < G::ELEMS) && static_cast<uint32_t>(gi) < unr &&
-                        static_cast<uint32_t>(gj) < un;
-        v[q] = ok ? in[off] : T(0);
-        if (CHECK && ok) loaded |= 1u << q;
-        c += DC;
-        gi += DR;
-        gj += DC;
-        off += DR * n + DC;
-        if (c >= G::SW) {
-            c -= G::SW;
-            gi += 1;
-            gj -= G::SW;
-            off += n - G::SW;
-        }
-    }
+    walk([&](int q, bool ok, int64_t off) { v[q] = ok ? in[off] : T(0); });  // all loads before the stores
     auto store = [&](auto f) {
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
@@ -147,28 +149,42 @@ __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const v
         }
     };
     if constexpr (CHECK) {
-        tile::IntCheck check;
-        if (i0 >= R && j0 >= G::RA && i0 - R + G::SH <= nr && j0 - G::RA + G::SW <= n) {  // every element loaded
-            store([&](int q) {
-                const float u = __fsub_rn(v[q], it.ref);
-                if ((q + 1) * tile::THREADS <= G::ELEMS || threadIdx.x + q * tile::THREADS < G::ELEMS) check.add(v[q], u);
-                return u;
-            });
-        } else {
-            store([&](int q) {
-                const float u = __fsub_rn(v[q], it.ref);
-                if (loaded >> q & 1u) check.add(v[q], u);
-                return u;
-            });
-        }
         it.known = true;
-        it.sums = check.sums<P, R>(it.ref, nsteps);
-        if (it.sums) return it;
-        it.ref = 0.0f;
+        if (tile::whole_f32(it.ref) && tile::whole_f32(corner)) {  // block-uniform
+            tile::IntCheck check;
+            if (i0 >= R && j0 >= G::RA && i0 - R + G::SH <= nr && j0 - G::RA + G::SW <= n) {  // all in the arrays
+#pragma unroll
+                for (int q = 0; q < PER; ++q)
+                    if ((q + 1) * tile::THREADS <= G::ELEMS || threadIdx.x + q * tile::THREADS < G::ELEMS)
+                        check.add(v[q], __fsub_rn(v[q], it.ref));
+            } else {
+                walk([&](int q, bool ok, int64_t) {
+                    if (ok) check.add(v[q], __fsub_rn(v[q], it.ref));
+                });
+            }
+            it.sums = check.sums<P, R>(it.ref, nsteps);
+        }
+        if (!it.sums) it.ref = 0.0f;
+        store([&](int q) { return __fsub_rn(v[q], it.ref); });
+    } else {
+        store([&](int q) { return v[q]; });
     }
-    store([&](int q) { return v[q]; });
     __syncthreads();
     return it;
+}
+
+// The FP32C tile at (i0, j0), staged and evaluated. A call: these families hold five stencils, and inlined
+// their routes kept one another's values alive and spilled (128 registers and 452 bytes for the stars' whole
+// run; as calls 80 registers). The row-by-row alignment check of the stores stands in for g.vec_ok.
+template <int P, int R, int STEPS>
+__device__ __noinline__ void item_fp32c(int64_t n, int64_t i0, int64_t j0, void* in_cur, void* in_nxt, void* out, int depth)
+{
+    using C = tile::Cfg<FP32C>;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const tile::IntTile it = stage_tile<P, R, FP32C, STEPS>(smem, in_cur, n, n, i0, j0, n, STEPS > 0 ? STEPS : depth);
+    tile::process_tile<P, R, FP32C, STEPS, tile::OUT_HBM>(smem, nullptr, i0, j0, n,
+                                                          tile::tile_has_out(i0, j0, n, R, C::TW, C::TH), in_nxt, out,
+                                                          false, depth, 0, n, nullptr, it);
 }
 
 // One work item: load the tile of grid g at `parity`, then evaluate it. tbl: the table area.
@@ -184,11 +200,15 @@ __device__ __forceinline__ void item(unsigned char* smem, int* s_red, const Grid
     // local memory)
     void* const in_cur = parity ? g.in[1] : g.in[0];
     void* const in_nxt = parity ? g.in[0] : g.in[1];
-    const int nsteps = STEPS > 0 ? STEPS : depth;
-    const tile::IntTile it = stage_tile<P, R, DT, STEPS>(smem, in_cur, n, n, i0, j0, n, nsteps);
-    tile::process_tile<P, R, DT, STEPS, tile::OUT_HBM>(smem, s_red, i0, j0, n, tile::tile_has_out(i0, j0, n, R, C::TW, C::TH),
-                                               in_nxt, g.out, g.vec_ok != 0, depth, 0, n,
-                                               tile::table_route<P, R, DT>() ? tbl : nullptr, it);
+    if constexpr (DT == FP32C) {
+        item_fp32c<P, R, STEPS>(n, i0, j0, in_cur, in_nxt, g.out, depth);
+    } else {
+        stage_tile<P, R, DT, STEPS>(smem, in_cur, n, n, i0, j0, n, 0);
+        tile::process_tile<P, R, DT, STEPS, tile::OUT_HBM>(smem, s_red, i0, j0, n,
+                                                           tile::tile_has_out(i0, j0, n, R, C::TW, C::TH), in_nxt, g.out,
+                                                           g.vec_ok != 0, depth, 0, n,
+                                                           tile::table_route<P, R, DT>() ? tbl : nullptr);
+    }
 }
 
 template <int DT, int STEPS, int FAM>
@@ -207,8 +227,18 @@ __device__ __forceinline__ void dispatch(unsigned char* smem, int* s_red, const 
 #undef PRK_ITEM
 }
 
+// CTAs per SM the register budget is cut for. FP32C: three for the stars and for the grids in launches of
+// one and two applications, which wait for their tiles' loads (48 grids of each pattern, 16 applications
+// and the warm-up, ms against two: stars one at a time 3.32 against 4.06, grids 5.64 against 6.36 on reals);
+// two for the grids' deeper launches (3.22 against 3.33 in eights).
 template <int DT, int STEPS, int FAM>
-__global__ void __launch_bounds__(tile::THREADS, 2)
+constexpr int batch_min_blocks()
+{
+    return FAM == FAM_F32_STAR || (FAM == FAM_F32_GRID && (STEPS == 1 || STEPS == 2)) ? 3 : 2;
+}
+
+template <int DT, int STEPS, int FAM>
+__global__ void __launch_bounds__(tile::THREADS, batch_min_blocks<DT, STEPS, FAM>())
     k_batch(const GridDesc* __restrict__ grids, const int64_t* __restrict__ tile_off, int ngrids, int64_t total,
             unsigned long long* __restrict__ queue, int parity, int depth)
 {

@@ -1793,6 +1793,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                                              unsigned char* tbl, const IntTile& pre = IntTile{})
 {
     const int nsteps = STEPS > 0 ? STEPS : (STEPS == OPERATOR ? 1 : depth);
+    constexpr bool ROUTE = int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>();
     using G = Geo<DT, R, TH_>;
     using C = Cfg<DT, TH_>;
     using T = typename C::T;
@@ -1832,6 +1833,31 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         }
 #pragma unroll
         for (int k = 0; k < CPT; ++k) o[k] = load_out(r, k);
+    };
+
+    // the same words as FP32C pairs
+    auto load_pairs = [&](int r, float (&hi)[CPT], float (&lo)[CPT]) {
+        const float2* src = OUT_SRC == OUT_SMEM
+                                ? reinterpret_cast<const float2*>(o_tile) + r * C::TW + c0
+                                : static_cast<const float2*>(static_cast<const void*>(out_v)) + (i0 + r) * n + gj;
+        if (OUT_SRC == OUT_SMEM || (gj + CPT <= n && (reinterpret_cast<uintptr_t>(src) & 15u) == 0)) {
+#pragma unroll
+            for (int k = 0; k < CPT; k += 2) {
+                const float4 w = *reinterpret_cast<const float4*>(src + k);
+                hi[k] = w.x;
+                lo[k] = w.y;
+                hi[k + 1] = w.z;
+                lo[k + 1] = w.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < CPT; ++k)
+                if (gj + k < n) {
+                    const float2 w = src[k];
+                    hi[k] = w.x;
+                    lo[k] = w.y;
+                }
+        }
     };
 
     // ---- FP64 power-of-two stencils: certify the tile for an exact route ----
@@ -2005,7 +2031,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
     // ---- FP32C: whole-number tiles of small range take the integer route ----
     int sums = 0;  // applications one FP32 sum takes on the route
     float uref = 0.0f;
-    if constexpr (int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>()) {
+    if constexpr (ROUTE) {
         if (pre.known) {
             sums = pre.sums;
             uref = pre.ref;
@@ -2016,28 +2042,30 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             const int rm = static_cast<int>(min(static_cast<int64_t>(G::SH / 2), row_hi - 1 - (i0 - R)));
             const int cm = static_cast<int>(min(static_cast<int64_t>(G::SW / 2), n - 1 - (j0 - G::RA)));
             uref = s_in[rm * G::SW + cm];
-            float4 u[PER];
-            IntCheck check;
-#pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int v = threadIdx.x + q * THREADS;
-                u[q] = v < NV ? reinterpret_cast<const float4*>(s_in)[v] : make_float4(uref, uref, uref, uref);
-                float* e = reinterpret_cast<float*>(&u[q]);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float x = e[k];
-                    e[k] = __fsub_rn(x, uref);
-                    if (!edge || inside(4 * v + k)) check.add(x, e[k]);
-                }
-            }
-            sums = check.sums<P, R>(uref, nsteps);
-            if (sums) {
+            if (whole_f32(uref) && whole_f32(s_in[R * G::SW + G::RA])) {  // block-uniform
+                float4 u[PER];
+                IntCheck check;
 #pragma unroll
                 for (int q = 0; q < PER; ++q) {
                     const int v = threadIdx.x + q * THREADS;
-                    if (v < NV) reinterpret_cast<float4*>(s_in)[v] = u[q];
+                    u[q] = v < NV ? reinterpret_cast<const float4*>(s_in)[v] : make_float4(uref, uref, uref, uref);
+                    float* e = reinterpret_cast<float*>(&u[q]);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float x = e[k];
+                        e[k] = __fsub_rn(x, uref);
+                        if (!edge || inside(4 * v + k)) check.add(x, e[k]);
+                    }
                 }
-                __syncthreads();
+                sums = check.sums<P, R>(uref, nsteps);
+                if (sums) {
+#pragma unroll
+                    for (int q = 0; q < PER; ++q) {
+                        const int v = threadIdx.x + q * THREADS;
+                        if (v < NV) reinterpret_cast<float4*>(s_in)[v] = u[q];
+                    }
+                    __syncthreads();
+                }
             }
         }
     }
@@ -2153,10 +2181,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             for (int k = 0; k < CPT; ++k) {
                 float oh = __uint_as_float(static_cast<uint32_t>(o[k]));
                 float ol = __uint_as_float(static_cast<uint32_t>(o[k] >> 32));
-                if constexpr (one_application(STEPS))
-                    df_add(oh, ol, sh[k], sl[k]);
-                else  // out stays in registers: renormalised once, before it is stored
-                    df_add_lazy(oh, ol, sh[k], sl[k]);
+                df_add(oh, ol, sh[k], sl[k]);
                 o[k] = static_cast<uint64_t>(__float_as_uint(oh)) | (static_cast<uint64_t>(__float_as_uint(ol)) << 32);
             }
         }
@@ -2306,10 +2331,27 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                 }
             }
         }
-        float si[int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>() ? ROWS : 1][CPT] = {};  // M * S of the thread's points (integer route)
-        if constexpr (int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>()) {
-            if (inted && has_out)
-                int_rows<P, R, CPT, ROWS, G::RA>(s_in + (warp * ROWS + R) * G::SW + G::RA + c0, G::SW, si);
+        if constexpr (ROUTE) {
+            if (inted) {  // a loop of its own, so that neither route's registers burden the other
+                float si[ROWS][CPT] = {};  // M * S of the thread's points
+                if (has_out)
+                    int_rows<P, R, CPT, ROWS, G::RA>(s_in + (warp * ROWS + R) * G::SW + G::RA + c0, G::SW, si);
+#pragma unroll
+                for (int rr = 0; rr < ROWS; ++rr) {
+                    const int r = warp * ROWS + rr;
+                    const int64_t gi = i0 + r, gg = gi + goff;
+                    if (!col_ok || gi >= row_end) continue;
+                    const bool row_out = has_out && gg >= R && gg < n - R;
+                    uint64_t o[CPT];
+                    if (row_out) {
+                        load_out_row(r, o);
+#pragma unroll
+                        for (int k = 0; k < CPT; ++k) int_add<P, R>(o[k], si[rr][k], 0.0f);
+                    }
+                    store_row(r, o, row_out);
+                }
+                return;
+            }
         }
 #pragma unroll
         for (int rr = 0; rr < ROWS; ++rr) {
@@ -2325,82 +2367,124 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
                 } else {
                     load_out_row(r, o);
                 }
-                if constexpr (int_route<P, R, DT, STEPS, OUT_SRC != OUT_SMEM>()) {
-                    if (inted) {
-#pragma unroll
-                        for (int k = 0; k < CPT; ++k) int_add<P, R>(o[k], si[rr][k], 0.0f);
-                    }
-                }
-                if (!tbl_done && !inted) apply_row(r, o);
+                if (!tbl_done) apply_row(r, o);
             }
             store_row(r, o, row_out);
         }
-    } else {
-        static_assert(G::ELEMS % 4 == 0, "the in-place advance moves 16-byte vectors");
-        if constexpr (DT == FP32C) {
-            if (inted) {
-                // The integer route: M * S of every application summed exactly, out read and updated once
-                // at the end. `sums` applications fit the FP32 sum; it then goes to an integer.
-                // The in += 1 of the thread's own points from the values its sums have just read, the halo beside
-                // them; a pass over the whole tile where the extra registers cost more (n=8192, whole runs,
-                // us per application: star R=1 47 to 43, R=2 51 to 48; launches of eight, R=5 85 to 88).
-                constexpr bool FUSED_ADVANCE = P == STAR && R <= 2;
-                float a[ROWS][CPT] = {};
-                int acc[ROWS][CPT] = {};
-                int held = 0;
+    } else if constexpr (DT == FP32C) {
+        static_assert(G::ELEMS % 4 == 0 && ROUTE, "the in-place advance moves 16-byte vectors");
+        if (inted) {
+            // The integer route: M * S of every application summed exactly, out read and updated once
+            // at the end. `sums` applications fit the FP32 sum; it then goes to an integer.
+            // The in += 1 of the thread's own points from the values its sums have just read, the halo beside
+            // them; a pass over the whole tile where the extra registers cost more (n=8192, whole runs,
+            // us per application: star R=1 47 to 43, R=2 51 to 48; launches of eight, R=5 85 to 88).
+            constexpr bool FUSED_ADVANCE = P == STAR && R <= 2;
+            float a[ROWS][CPT] = {};
+            int acc[ROWS][CPT] = {};
+            int held = 0;
 #pragma unroll 1
-                for (int t = 0; t < nsteps; ++t) {
-                    if (held == sums) {
-                        held = 0;
+            for (int t = 0; t < nsteps; ++t) {
+                if (held == sums) {
+                    held = 0;
 #pragma unroll
-                        for (int rr = 0; rr < ROWS; ++rr)
-#pragma unroll
-                            for (int k = 0; k < CPT; ++k) {
-                                acc[rr][k] += __float2int_rn(a[rr][k]);
-                                a[rr][k] = 0.0f;
-                            }
-                    }
-                    ++held;
-                    float* const mine = s_in + (warp * ROWS + R) * G::SW + G::RA + c0;
-                    float own[ROWS][CPT];
-                    if (has_out) int_rows<P, R, CPT, ROWS, G::RA>(mine, G::SW, a, FUSED_ADVANCE ? own : nullptr);
-                    if (t + 1 < nsteps) {  // in += 1
-                        __syncthreads();
-                        if (FUSED_ADVANCE && has_out) {
-#pragma unroll
-                            for (int rr = 0; rr < ROWS; ++rr) {
-#pragma unroll
-                                for (int k = 0; k < CPT; ++k) own[rr][k] = __fadd_rn(own[rr][k], 1.0f);
-                                st_vec(mine + rr * G::SW, own[rr]);
-                            }
-                            advance_halo_f32<G::SW, G::SH, R, G::RA>(s_in, s_in);
-                        } else {
-                            advance_f32<G::ELEMS>(s_in);
-                        }
-                        __syncthreads();
-                    }
-                }
-#pragma unroll
-                for (int rr = 0; rr < ROWS; ++rr) {
-                    const int r = warp * ROWS + rr;
-                    const int64_t gi = i0 + r, gg = gi + goff;
-                    if (!col_ok || gi >= row_end) continue;
-                    const bool row_out = has_out && gg >= R && gg < n - R;
-                    uint64_t o[CPT];
-                    if (row_out) {
-                        load_out_row(r, o);
+                    for (int rr = 0; rr < ROWS; ++rr)
 #pragma unroll
                         for (int k = 0; k < CPT; ++k) {
-                            const int t = acc[rr][k] + __float2int_rn(a[rr][k]);
-                            const float th = __int2float_rn(t);
-                            int_add<P, R>(o[k], th, __int2float_rn(t - __float2int_rn(th)));
+                            acc[rr][k] += __float2int_rn(a[rr][k]);
+                            a[rr][k] = 0.0f;
                         }
-                    }
-                    store_row(r, o, row_out);
                 }
-                return;
+                ++held;
+                float* const mine = s_in + (warp * ROWS + R) * G::SW + G::RA + c0;
+                float own[ROWS][CPT];
+                if (has_out) int_rows<P, R, CPT, ROWS, G::RA>(mine, G::SW, a, FUSED_ADVANCE ? own : nullptr);
+                if (t + 1 < nsteps) {  // in += 1
+                    __syncthreads();
+                    if (FUSED_ADVANCE && has_out) {
+#pragma unroll
+                        for (int rr = 0; rr < ROWS; ++rr) {
+#pragma unroll
+                            for (int k = 0; k < CPT; ++k) own[rr][k] = __fadd_rn(own[rr][k], 1.0f);
+                            st_vec(mine + rr * G::SW, own[rr]);
+                        }
+                        advance_halo_f32<G::SW, G::SH, R, G::RA>(s_in, s_in);
+                    } else {
+                        advance_f32<G::ELEMS>(s_in);
+                    }
+                    __syncthreads();
+                }
+            }
+#pragma unroll
+            for (int rr = 0; rr < ROWS; ++rr)
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) acc[rr][k] += __float2int_rn(a[rr][k]);
+#pragma unroll
+            for (int rr = 0; rr < ROWS; ++rr) {
+                const int r = warp * ROWS + rr;
+                const int64_t gi = i0 + r, gg = gi + goff;
+                if (!col_ok || gi >= row_end) continue;
+                const bool row_out = has_out && gg >= R && gg < n - R;
+                uint64_t o[CPT];
+                if (row_out) {
+                    load_out_row(r, o);
+#pragma unroll
+                    for (int k = 0; k < CPT; ++k) {
+                        const int t = acc[rr][k];
+                        const float th = __int2float_rn(t);
+                        int_add<P, R>(o[k], th, __int2float_rn(t - __float2int_rn(th)));
+                    }
+                }
+                store_row(r, o, row_out);
+            }
+            return;
+        }
+        // The group sums: out stays in registers, accumulated without renormalising. As floats, not in the
+        // loop of FP64 words below: there the two routes together spilled (n=8192, real values, eight
+        // applications, us per application: star R=4 151 to 141, grid R=4 377 to 330; on the loop of
+        // words without the integer route 144 and 353).
+        float oh[ROWS][CPT], ol[ROWS][CPT];
+        bool ract[ROWS];  // the row holds interior points
+#pragma unroll
+        for (int rr = 0; rr < ROWS; ++rr) {
+            const int r = warp * ROWS + rr;
+            const int64_t gi = i0 + r, gg = gi + goff;
+            ract[rr] = col_ok && gi < row_end && has_out && gg >= R && gg < n - R;
+#pragma unroll
+            for (int k = 0; k < CPT; ++k) oh[rr][k] = ol[rr][k] = 0.0f;
+            if (ract[rr]) load_pairs(r, oh[rr], ol[rr]);
+        }
+#pragma unroll 1
+        for (int t = 0; t < nsteps; ++t) {
+            if (t > 0) {  // in += 1 over the whole tile, halo included
+                __syncthreads();
+                advance_f32<G::ELEMS>(s_in);
+                __syncthreads();
+            }
+#pragma unroll
+            for (int rr = 0; rr < ROWS; ++rr) {
+                if (!ract[rr]) continue;
+                float sh[CPT], sl[CPT];
+                fp32c_points<P, R, CPT, G::RA>(s_in + (warp * ROWS + rr + R) * G::SW + G::RA + c0, G::SW, sh, sl);
+#pragma unroll
+                for (int k = 0; k < CPT; ++k) df_add_lazy(oh[rr][k], ol[rr][k], sh[k], sl[k]);
             }
         }
+#pragma unroll
+        for (int rr = 0; rr < ROWS; ++rr) {
+            const int r = warp * ROWS + rr;
+            if (!col_ok || i0 + r >= row_end) continue;
+            uint64_t o[CPT];
+#pragma unroll
+            for (int k = 0; k < CPT; ++k) {
+                float h, l;
+                fast_two_sum(oh[rr][k], ol[rr][k], h, l);
+                o[k] = static_cast<uint64_t>(__float_as_uint(h)) | (static_cast<uint64_t>(__float_as_uint(l)) << 32);
+            }
+            store_row(r, o, ract[rr]);
+        }
+    } else {
+        static_assert(G::ELEMS % 4 == 0, "the in-place advance moves 16-byte vectors");
         // out of the thread's points stays in registers across the applications
         uint64_t o[ROWS][CPT];
         bool ract[ROWS];  // the row holds interior points
@@ -2496,27 +2580,23 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
         for (int t = 0; t < nsteps; ++t) {
             if (t > 0) {  // advance the whole tile, halo included: in_{k+1} = in_k + 1
                 __syncthreads();
-                if constexpr (DT == FP64) {
-                    bool adv = false;
-                    if constexpr (EXACT) {
-                        if (fexact) {
-                            advance_f32<G::ELEMS>(reinterpret_cast<float*>(s_in));
-                            adv = true;
-                        } else if (unit != fx::NOT_FIXED) {
-                            advance_i64<G::ELEMS>(reinterpret_cast<int64_t*>(s_in), 1ll << (-unit));
-                            adv = true;
-                        }
+                bool adv = false;
+                if constexpr (EXACT) {
+                    if (fexact) {
+                        advance_f32<G::ELEMS>(reinterpret_cast<float*>(s_in));
+                        adv = true;
+                    } else if (unit != fx::NOT_FIXED) {
+                        advance_i64<G::ELEMS>(reinterpret_cast<int64_t*>(s_in), 1ll << (-unit));
+                        adv = true;
                     }
-                    if constexpr (!EXACT) {
-                        if (iwhole) {
-                            advance_i32<G::ELEMS>(reinterpret_cast<int32_t*>(s_in));
-                            adv = true;
-                        }
-                    }
-                    if (!adv) advance_f64<G::ELEMS>(s_in);
-                } else {
-                    advance_f32<G::ELEMS>(s_in);
                 }
+                if constexpr (!EXACT) {
+                    if (iwhole) {
+                        advance_i32<G::ELEMS>(reinterpret_cast<int32_t*>(s_in));
+                        adv = true;
+                    }
+                }
+                if (!adv) advance_f64<G::ELEMS>(s_in);
                 __syncthreads();
             }
             if constexpr (PLANES) {
@@ -2534,18 +2614,6 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             for (int rr = 0; rr < ROWS; ++rr)
                 if (ract[rr]) apply_row(warp * ROWS + rr, o[rr]);
         }
-        }
-        if constexpr (DT == FP32C) {  // the pairs accumulated without renormalising
-#pragma unroll
-            for (int rr = 0; rr < ROWS; ++rr)
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    float oh, ol;
-                    fast_two_sum(__uint_as_float(static_cast<uint32_t>(o[rr][k])),
-                                 __uint_as_float(static_cast<uint32_t>(o[rr][k] >> 32)), oh, ol);
-                    o[rr][k] = static_cast<uint64_t>(__float_as_uint(oh)) |
-                               (static_cast<uint64_t>(__float_as_uint(ol)) << 32);
-                }
         }
         if (oint) {
 #pragma unroll
@@ -2583,11 +2651,16 @@ constexpr int min_blocks()
         constexpr int fit = SMEM_PER_SM / (tile_smem<P, R, DT, TH_>() + 1024);
         return fit < 3 ? 2 : (fit < strict_tiles<P, R>() ? fit : strict_tiles<P, R>());
     }
-    // FP32C grid R >= 3: three tiles per SM (80 registers; n=8192, the integer route, us per application
-    // against two tiles: grid R=3 263 against 300 at one application, 100 against 105 in whole runs; R=5
-    // 420 against 446 and 222 against 228). The group sums of tiles off that route would want the
-    // registers of two.
-    if (DT == FP32C && P == GRID && R >= 3) return Geo<DT, R, TH_>::CTAS < 3 ? Geo<DT, R, TH_>::CTAS : 3;
+    // FP32C grid R >= 3: three tiles per SM (80 registers). n=8192, us per application against two tiles, one
+    // application: grid R=3 257 against 303 on whole numbers and 286 against 369 on reals, R=5 376 against
+    // 432 and 560 against 596; whole runs: R=4 150 against 155 and 332 against 337. The group sums of grid
+    // R=5 hold 72 values per thread and want the registers of two tiles in several applications (whole
+    // runs: 502 against 550 on reals, 227 against 219 on whole numbers; launches of two do not, 531 and 523
+    // on reals, 305 and 335).
+    if (DT == FP32C && P == GRID && R >= 3) {
+        constexpr int most = R == 5 && !one_application(STEPS) && STEPS != 2 ? 2 : 3;
+        return Geo<DT, R, TH_>::CTAS < most ? Geo<DT, R, TH_>::CTAS : most;
+    }
     const int b = Geo<DT, R, TH_>::CTAS;
     if (one_application(STEPS)) return b;
     const int cap = DT == FP64 ? 4 : 3;  // FP64 power-of-two: the FP32 route is shared-memory bound

@@ -1,0 +1,100 @@
+"""FP32C on fields of real numbers, whose tiles keep the group sums beside the integer route: right at every
+form of launch, tile and batch, with the values the tiles ask first (the middle one and the first) whole
+or not, and no slower for the route that they do not take."""
+import statistics
+
+import numpy as np
+import pytest
+
+import kernels_gb300 as kg
+from oracle import prk_oracle as po
+
+pytestmark = pytest.mark.gpu
+
+ALL = [(p, r) for p in (kg.STAR, kg.GRID) for r in range(1, 6)]
+
+
+def exact(pattern, r, a, apps):
+    """apps applications in binary64 on the FP32 values of `in` (which rounds as it grows), and the
+    sum of |w d| over the taps' differences d."""
+    n = a.shape[0]
+    s = np.zeros((n - 2 * r, n - 2 * r), np.float64)
+    m = np.zeros_like(s)
+    x = a.copy()
+    for _ in range(apps):
+        for dc, dr, w in po.taps(pattern, r):
+            if w > 0:
+                d = x[r + dr:n - r + dr, r + dc:n - r + dc].astype(np.float64) - x[r - dr:n - r - dr, r - dc:n - r - dc]
+                s += d / np.float64(round(1.0 / w))
+                m += np.abs(d) / np.float64(round(1.0 / w))
+        x += np.float32(1.0)
+    return s, m, x
+
+
+@pytest.mark.parametrize("pattern,r", ALL)
+@pytest.mark.parametrize("n", [180, 149])
+@pytest.mark.parametrize("kind", ["real", "whole where asked"])
+def test_every_form(cuda, pattern, r, n, kind):
+    rng = np.random.default_rng(10 * r + pattern)
+    a = rng.uniform(-40.0, 40.0, (n, n)).astype(np.float32)
+    if kind != "real":  # every 32-row tile's first value, and the block around its middle
+        a[::32, ::128] = np.round(a[::32, ::128])
+        for i in range(0, n, 32):
+            for j in range(0, n, 128):
+                a[i + 8:i + 24, j + 40:j + 90] = np.round(a[i + 8:i + 24, j + 40:j + 90])
+    out0 = np.zeros((n, n, 2), np.float32)
+    out0[..., 0] = rng.uniform(-50.0, 50.0, (n, n))
+    taps = sum(1 for *_, w in po.taps(pattern, r) if w > 0)
+    inner = (slice(r, n - r), slice(r, n - r))
+
+    def fresh():
+        in_ = cuda.from_numpy(a.copy()).cuda()
+        return in_, cuda.empty_like(in_), cuda.from_numpy(out0.copy()).cuda()
+
+    def check(out, apps, in_end):
+        s, m, x = exact(pattern, r, a, apps)
+        got = out.cpu().numpy().astype(np.float64)
+        err = np.abs(got[inner].sum(axis=-1) - (out0[inner][..., 0] + s))
+        # a difference and each add to its group's sum round to 24 bits of what no sum of the group's
+        # differences exceeds; products and two-float sums to 2^-44 of theirs
+        bound = m * np.float64((taps + 1) * 2.0 ** -24) + (m + np.abs(out0[inner][..., 0])) * np.float64(2.0 ** -44)
+        assert (err <= bound).all(), (apps, float((err / bound).max()))
+        assert in_end is None or np.array_equal(in_end.cpu().numpy(), x)
+
+    apps = 6
+    for kw in ({"depth": 1}, {"depth": 2}, {"depth": 4}, {"whole": True}, *([{"depth": 4, "tall": True}] if n % 4 == 0 else [])):
+        in_a, in_b, out = fresh()
+        res = kg.run(pattern, r, apps - 1, in_a, in_b, out, **kw)
+        check(out, apps, res.final_in)
+    for kw in ({"depth": 1}, {"depth": 2}, {"depth": 4}, {"whole": True}):
+        in_a, in_b, out = fresh()
+        batch = kg.Batch([(pattern, r, in_a, in_b, out)], **kw)
+        batch.run(apps - 1)
+        check(out, apps, batch.final_in(0))
+    in_a, _, out = fresh()
+    kg.apply(pattern, r, in_a, out)
+    check(out, 1, None)
+
+
+@pytest.mark.parametrize("pattern,r,most", [(kg.STAR, 5, 1.1), (kg.GRID, 3, 1.25)])
+def test_reals_do_not_pay_for_the_integer_route(cuda, pattern, r, most):
+    """One fused application at n=8192 on reals against whole numbers. Paying for the check and for a shared
+    register allocation, the reals took 1.18 (star R=5) and 1.46 times as long; 1.00 and 1.11 without."""
+    in_a, in_b, out = kg.alloc(8192, kg.FP32C)
+
+    def time():
+        ts = []
+        for _ in range(9):
+            e = [cuda.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            for _ in range(4):
+                kg.apply(pattern, r, in_a, out, in_b)
+            e[1].record()
+            cuda.cuda.synchronize()
+            ts.append(e[0].elapsed_time(e[1]))
+        return statistics.median(ts)
+
+    kg.init(in_a, out)
+    whole = time()
+    in_a.copy_(cuda.rand_like(in_a))
+    assert time() <= most * whole
