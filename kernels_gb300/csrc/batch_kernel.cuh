@@ -150,7 +150,7 @@ __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const v
     };
     if constexpr (CHECK) {
         it.known = true;
-        if (tile::whole_f32(it.ref) && tile::whole_f32(corner)) {  // block-uniform
+        if (tile::IntCheck::hopeful<P, R>(it.ref, corner)) {  // block-uniform
             tile::IntCheck check;
             if (i0 >= R && j0 >= G::RA && i0 - R + G::SH <= nr && j0 - G::RA + G::SW <= n) {  // all in the arrays
 #pragma unroll

@@ -448,6 +448,13 @@ __device__ __forceinline__ bool whole_f32(float x) { return __fsub_rn(__fadd_rn(
 struct IntCheck {
     bool whole = true;
     float most = 0.0f;
+    // Whether two of the tile's values let it take the route, asked before all of them are: a tile of reals
+    // or of whole numbers far apart then does without the check and its vote.
+    template <int P, int R>
+    static __device__ __forceinline__ bool hopeful(float ref, float v)
+    {
+        return whole_f32(ref) && whole_f32(v) && fabsf(__fsub_rn(v, ref)) < static_cast<float>(int_wide<P, R>());
+    }
     __device__ __forceinline__ void add(float v, float u)
     {
         whole = whole && whole_f32(v);
@@ -2042,7 +2049,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             const int rm = static_cast<int>(min(static_cast<int64_t>(G::SH / 2), row_hi - 1 - (i0 - R)));
             const int cm = static_cast<int>(min(static_cast<int64_t>(G::SW / 2), n - 1 - (j0 - G::RA)));
             uref = s_in[rm * G::SW + cm];
-            if (whole_f32(uref) && whole_f32(s_in[R * G::SW + G::RA])) {  // block-uniform
+            if (IntCheck::hopeful<P, R>(uref, s_in[R * G::SW + G::RA])) {  // block-uniform
                 float4 u[PER];
                 IntCheck check;
 #pragma unroll
