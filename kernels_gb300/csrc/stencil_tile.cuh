@@ -1124,8 +1124,9 @@ __device__ __forceinline__ void build_tables(uint64_t* T64, uint4* T96, int base
     }
 }
 
-// Where a row of the table route's points lies: a row whose points are all outside the interior or
-// past row_end is skipped (row-uniform); a column outside the interior is computed and dropped.
+// Whether a row of the table route's tile holds points to update (row-uniform). The 96-bit form skips the
+// other rows; the narrow form takes a thread's eight points together and drops those outside, and skips a
+// warp's rows only where none has any.
 __device__ __forceinline__ bool table_row_active(bool has_out, int64_t gi, int64_t gg, int64_t row_end, int64_t n, int R)
 {
     return has_out && gi < row_end && gg >= R && gg < n - R;
@@ -1144,7 +1145,7 @@ __device__ __forceinline__ bool table_row_active(bool has_out, int64_t gi, int64
 //    the leading bit, no per-point masks. The other taps find it per point (bfind).
 // Over the tiles of a PRK field at n=16384, 96% of the taps of star R=3 and 93% of grid R=5's have one
 // rounding position; at n=4096 88% and 78%. Windows that hold zero, or span too many binades, take the
-// 96-bit form (table_chain).
+// 96-bit form (table_rows).
 //
 // A tap is a loop iteration over eight points of a thread, which share its constants and descriptor, so
 // the code stays small at 110 taps; the tile holds table offsets instead of values, so a point's two
@@ -1381,51 +1382,69 @@ __device__ __forceinline__ void narrow_chain(const int32_t* sp, const unsigned c
     }
 }
 
-// The chains of four points in 96-bit fixed point: rows r and r + WARPS (q >> 1) of columns c and c + 32
-// (q & 1); sp points at (r, c) of the int32 tile, the tables cover [base, base + TBL_L). The adds of the
-// first fixed_taps<P, R, ONE>() taps run in fixed point (fx::fx96_acc_round), the rest on the binary64
-// pipe. A tap is a loop iteration, as in the narrow form: windows that take this form are few (those
-// that hold zero), and unrolled taps cost every kernel of the stencil registers and code. A rounded sum
-// is -0 only when every term is -0: no positive weight and no value but zero so far.
-template <int P, int R, int SW, bool ONE>
-__device__ __forceinline__ void table_chain(const int32_t* sp, const unsigned char* tbl, int base, double (&d)[4])
+// True when a positive weight lies among the fixed taps: then the fixed part never sums to -0 (a rounded sum
+// is -0 only when every term is -0, and w * v with w > 0 is never -0).
+template <int P, int R, bool ONE>
+constexpr bool fixed_prefix_has_positive()
 {
-    constexpr int N = tap_count(P, R), KF = fixed_taps<P, R, ONE>(), NG = group_count<P, R>(), NQ = 4;
-    const auto& T = c_narrow<P, R, SW>;
-    uint32_t x[NQ][3] = {};
-    int anyv[NQ] = {};
-    bool positive = false;
-    auto value = [&](const int32_t* s, int q) { return s[(q >> 1) * WARPS * SW + 32 * (q & 1)]; };
+    constexpr StrictTaps<P, R> t = make_strict_taps<P, R>();
+    for (int k = 0; k < fixed_taps<P, R, ONE>(); ++k)
+        if (!t.neg[k]) return true;
+    return false;
+}
+
+// The 96-bit form: out += the chains of columns c and c + 32 of every WARPS-th row from r on, for the rows and
+// columns whose bits are set. `point`, `out` and `tbl`: shared-memory addresses of the int32 tile's and the
+// out words' (r, c), and of the tables, which cover [base, base + TBL_L). The adds of the first
+// fixed_taps<P, R, ONE>() taps run in fixed point (fx::fx96_acc_round), the rest on the binary64 pipe.
+// Bound by the integer ALU, so the taps are unrolled, with their offsets and signs in the instructions; as a
+// loop over the taps, values about zero, n=4096, us per application: star R=5 in launches of two 450
+// against 411, grid R=3 855 against 770, star R=3 on 64-row tiles 293 against 247. A call, because the windows
+// that take this form are few and inlined it cost every kernel of the stencil registers and code (the call
+// costs star R=3, 4 up to 2% at one application, n=16384, PRK field: 2533 to 2578 us, 2938 to 2999).
+template <int P, int R, int SW, int TW, bool ONE>
+__device__ __noinline__ void table_rows(uint32_t point, uint32_t out, uint32_t tbl, int base, uint32_t rows, uint32_t cols)
+{
+    constexpr StrictTaps<P, R> TP = make_strict_taps<P, R>();
+    constexpr int N = tap_count(P, R), KF = fixed_taps<P, R, ONE>(), NG = group_count<P, R>();
+    constexpr bool POS = fixed_prefix_has_positive<P, R, ONE>();
+    const uint64_t* T64 = static_cast<const uint64_t*>(__cvta_shared_to_generic(tbl));
+    const uint4* T96 = static_cast<const uint4*>(__cvta_shared_to_generic(tbl + NG * TBL_L * 8));
 #pragma unroll 1
-    for (int t = 0; t < KF; ++t) {
-        const NarrowTap tp = T.tap[t];
-        const int32_t* s = sp + tp.off;
-        const unsigned char* tf = tbl + NG * TBL_L * 8 + 2 * tp.t64;
-        positive = positive || tp.sign == 0u;
+    for (; rows; rows >>= 1, point += WARPS * SW * 4, out += WARPS * TW * 8) {
+        if (!(rows & 1u)) continue;
+        const int32_t* sp = static_cast<const int32_t*>(__cvta_shared_to_generic(point));
+        uint32_t x[2][3] = {};
+        int anyv[2] = {};
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const int v = value(s, q);
-            anyv[q] |= v;
-            const uint4 p = *reinterpret_cast<const uint4*>(tf + (v - base) * 16);
-            if (tp.sign)
-                fx::fx96_acc_round<true>(x[q][0], x[q][1], x[q][2], p.x, p.y, p.z);
-            else
-                fx::fx96_acc_round<false>(x[q][0], x[q][1], x[q][2], p.x, p.y, p.z);
+        for (int t = 0; t < KF; ++t) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int v = sp[TP.dr[t] * SW + TP.dc[t] + 32 * h];
+                if (!POS) anyv[h] |= v;
+                const uint4 p = T96[TP.g[t] * TBL_L + (v - base)];
+                if (TP.neg[t])
+                    fx::fx96_acc_round<true>(x[h][0], x[h][1], x[h][2], p.x, p.y, p.z);
+                else
+                    fx::fx96_acc_round<false>(x[h][0], x[h][1], x[h][2], p.x, p.y, p.z);
+            }
         }
-    }
+        double d[2];
 #pragma unroll
-    for (int q = 0; q < NQ; ++q)
-        d[q] = as_dbl(fx::fx96_to_bits(x[q][0], x[q][1], x[q][2], !positive && anyv[q] == 0));
-#pragma unroll 1
-    for (int t = KF; t < N; ++t) {
-        const NarrowTap tp = T.tap[t];
-        const int32_t* s = sp + tp.off;
-        const unsigned char* tf = tbl + tp.t64;
+        for (int h = 0; h < 2; ++h) d[h] = as_dbl(fx::fx96_to_bits(x[h][0], x[h][1], x[h][2], !POS && anyv[h] == 0));
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const uint2 p = *reinterpret_cast<const uint2*>(tf + (value(s, q) - base) * 8);
-            d[q] = __dadd_rn(d[q], as_dbl((static_cast<uint64_t>(p.y ^ tp.sign) << 32) | p.x));
+        for (int t = KF; t < N; ++t) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int v = sp[TP.dr[t] * SW + TP.dc[t] + 32 * h];
+                const double p = as_dbl(T64[TP.g[t] * TBL_L + (v - base)]);
+                d[h] = TP.neg[t] ? __dsub_rn(d[h], p) : __dadd_rn(d[h], p);
+            }
         }
+        uint64_t* o = static_cast<uint64_t*>(__cvta_shared_to_generic(out));
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (cols >> h & 1u) o[32 * h] = as_bits(__dadd_rn(as_dbl(o[32 * h]), d[h]));
     }
 }
 
@@ -1721,19 +1740,17 @@ __device__ __forceinline__ bool table_tile(int32_t* si, uint64_t* o_s, uint64_t*
                 }
             }
         } else {
-            const int32_t* s0 = si + cur + R * SW + ((SW - TW) / 2);  // the tile's (0, 0)
-#pragma unroll 1
-            for (int rr = 0; rr < ROWS; rr += 2) {
-                const int r = warp + WARPS * rr;
-                double d[4];
-                table_chain<P, R, SW, ONE>(s0 + r * SW + lane, tbl, base, d);
+            uint32_t rows = 0, cols = 0;  // the warp's rows and columns that hold points to update
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int rq = r + (q >> 1) * WARPS, c = lane + 32 * (q & 1);
-                    if (table_row_active(has_out, i0 + rq, i0 + rq + goff, row_end, n, R) && j0 + c >= R && j0 + c < n - R)
-                        o_s[rq * TW + c] = as_bits(__dadd_rn(as_dbl(o_s[rq * TW + c]), d[q]));
-                }
+            for (int rr = 0; rr < ROWS; ++rr) {
+                const int64_t gi = i0 + warp + WARPS * rr;
+                if (table_row_active(has_out, gi, gi + goff, row_end, n, R)) rows |= 1u << rr;
             }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (j0 + lane + 32 * h >= R && j0 + lane + 32 * h < n - R) cols |= 1u << h;
+            table_rows<P, R, SW, TW, ONE>(smem_addr(si + cur + (warp + R) * SW + (SW - TW) / 2 + lane),
+                                          smem_addr(o_s + warp * TW + lane), smem_addr(tbl), base, rows, cols);
         }
         if (t + 1 < nsteps) {  // in += 1
             advance_i32_to<ELEMS>(si + cur, si + (ELEMS - cur), narrow ? 8 : 1);
