@@ -95,8 +95,8 @@ struct Layout {
 // Thread t takes elements t, t + THREADS, ... of the row-major tile; its row, column and grid offset
 // advance by constants from one element to the next (one division per thread, none per element).
 // FP32C: the values are checked for the integer route (tile::IntTile) in their registers and stored as the
-// tile's route wants them. The tile's middle and first values are asked first, by every thread: a field of
-// real numbers then pays for two loads, not for the check and a vote. row_hi: the first array row no point
+// tile's route wants them. Three of the tile's values are asked first, by every thread: a field of real numbers
+// then pays for their loads, not for the check and a vote. row_hi: the first array row no point
 // reads.
 template <int P, int R, int DT, int STEPS>
 __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const void* in_v, int64_t n, int64_t nr,
@@ -133,11 +133,12 @@ __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const v
     };
     tile::IntTile it;
     constexpr bool CHECK = tile::int_route<P, R, DT, STEPS, true>();
-    float corner = 0.0f;
-    if constexpr (CHECK) {  // the value nearest the tile's middle inside the grid, and the tile's first
+    float first = 0.0f, left = 0.0f;
+    if constexpr (CHECK) {  // the value nearest the tile's middle inside the grid, the tile's first, and its row's
         const int64_t rm = min(i0 - R + G::SH / 2, row_hi - 1), cm = min(j0 - G::RA + G::SW / 2, n - 1);
         it.ref = in[rm * n + cm];
-        corner = in[i0 * n + j0];
+        first = in[i0 * n + j0];
+        left = in[rm * n + j0];
     }
     T v[PER];
     walk([&](int q, bool ok, int64_t off) { v[q] = ok ? in[off] : T(0); });  // all loads before the stores
@@ -150,7 +151,7 @@ __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const v
     };
     if constexpr (CHECK) {
         it.known = true;
-        if (tile::IntCheck::hopeful<P, R>(it.ref, corner)) {  // block-uniform
+        if (tile::IntCheck::hopeful<P, R>(it.ref, first, left)) {  // block-uniform
             tile::IntCheck check;
             if (i0 >= R && j0 >= G::RA && i0 - R + G::SH <= nr && j0 - G::RA + G::SW <= n) {  // all in the arrays
 #pragma unroll

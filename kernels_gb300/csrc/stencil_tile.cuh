@@ -448,12 +448,13 @@ __device__ __forceinline__ bool whole_f32(float x) { return __fsub_rn(__fadd_rn(
 struct IntCheck {
     bool whole = true;
     float most = 0.0f;
-    // Whether two of the tile's values let it take the route, asked before all of them are: a tile of reals
+    // Whether three of the tile's values let it take the route, asked before all of them are: a tile of reals
     // or of whole numbers far apart then does without the check and its vote.
     template <int P, int R>
-    static __device__ __forceinline__ bool hopeful(float ref, float v)
+    static __device__ __forceinline__ bool hopeful(float ref, float v, float w)
     {
-        return whole_f32(ref) && whole_f32(v) && fabsf(__fsub_rn(v, ref)) < static_cast<float>(int_wide<P, R>());
+        const float far = fmaxf(fabsf(__fsub_rn(v, ref)), fabsf(__fsub_rn(w, ref)));
+        return whole_f32(ref) && whole_f32(v) && whole_f32(w) && far < static_cast<float>(int_wide<P, R>());
     }
     __device__ __forceinline__ void add(float v, float u)
     {
@@ -2053,7 +2054,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             const int rm = static_cast<int>(min(static_cast<int64_t>(G::SH / 2), row_hi - 1 - (i0 - R)));
             const int cm = static_cast<int>(min(static_cast<int64_t>(G::SW / 2), n - 1 - (j0 - G::RA)));
             uref = s_in[rm * G::SW + cm];
-            if (IntCheck::hopeful<P, R>(uref, s_in[R * G::SW + G::RA])) {  // block-uniform
+            if (IntCheck::hopeful<P, R>(uref, s_in[R * G::SW + G::RA], s_in[rm * G::SW + G::RA])) {  // block-uniform
                 float4 u[PER];
                 IntCheck check;
 #pragma unroll
@@ -2383,8 +2384,8 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             store_row(r, o, row_out);
         }
     } else if constexpr (DT == FP32C) {
-        static_assert(G::ELEMS % 4 == 0 && ROUTE, "the in-place advance moves 16-byte vectors");
-        if (inted) {
+        static_assert(G::ELEMS % 4 == 0, "the in-place advance moves 16-byte vectors");
+        if (ROUTE && inted) {
             // The integer route: M * S of every application summed exactly, out read and updated once
             // at the end. `sums` applications fit the FP32 sum; it then goes to an integer.
             // The in += 1 of the thread's own points from the values its sums have just read, the halo beside
