@@ -422,14 +422,17 @@ struct IntBound {
                   "integer route bounds");
 };
 
-// Launches that try the integer route: all on the TMA tiles (PLAIN false), where one fused application
-// is bound by HBM on either route and grid R >= 3 gains (n=8192, grid R=4: 419 to 327 us), so that a
-// result does not depend on the depth. On the plain-staged tiles, bound by issue, one fused application
-// of the others keeps the group sums (n=8189, star R=1: 274 us; 307 with the check while staging).
+// Launches that try the integer route: all on the TMA tiles (PLAIN false), where one fused application is
+// bound by HBM on either route and grid R >= 3 gains (n=8192, grid R=4: 373 to 300 us). On the plain-staged
+// and batched tiles one application of the others keeps the group sums, which cost it no check (n=8189, star
+// R=1: 274 us, 307 with the check), and so do the batched launches of two, four and eight of the stencils
+// with power-of-two weights (32 grids of star R=1, 2 and grid R=1 in twos: 791 against 954 us), whose group
+// sums of whole numbers are exact as well. Where the exact sum is no FP32 pair the last bits differ between
+// the routes, so there they may depend on the depth.
 template <int P, int R, int DT, int STEPS, bool PLAIN>
 __host__ __device__ constexpr bool int_route()
 {
-    return DT == FP32C && (!PLAIN || STEPS != 1 || (P == GRID && R >= 3));
+    return DT == FP32C && (!PLAIN || (STEPS > 0 ? (STEPS == 1 ? P == GRID && R >= 3 : !pow2_weights(P, R)) : true));
 }
 
 // Whether a staged FP32C tile takes the integer route, and its ref: checked while it was staged by plain
