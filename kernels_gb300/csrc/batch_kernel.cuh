@@ -94,8 +94,9 @@ struct Layout {
 // outside the arrays (nr rows of n columns), all loads issued before the first shared-memory store.
 // Thread t takes elements t, t + THREADS, ... of the row-major tile; its row, column and grid offset
 // advance by constants from one element to the next (one division per thread, none per element).
-// FP32C: the values are checked for the integer route (tile::IntTile) in their registers and stored as the
-// tile's route wants them. Three of the tile's values are asked first, by every thread: a field of real numbers
+// FP32C: the values are checked for the integer route (tile::IntTile) on their way from the registers and
+// stored as that route wants them, or as they are when some value fails; the barrier that ends the staging
+// collects the verdict, so the check adds no pass over the tile and no barrier. Three of the tile's values are asked first, by every thread: a field of real numbers
 // then pays for their loads, not for the check and a vote. row_hi: the first array row no point
 // reads.
 template <int P, int R, int DT, int STEPS>
@@ -154,19 +155,22 @@ __device__ __forceinline__ tile::IntTile stage_tile(unsigned char* smem, const v
         if (tile::IntCheck::hopeful<P, R>(it.ref, first, left)) {  // block-uniform
             tile::IntCheck check;
             if (i0 >= R && j0 >= G::RA && i0 - R + G::SH <= nr && j0 - G::RA + G::SW <= n) {  // all in the arrays
-#pragma unroll
-                for (int q = 0; q < PER; ++q)
-                    if ((q + 1) * tile::THREADS <= G::ELEMS || threadIdx.x + q * tile::THREADS < G::ELEMS)
-                        check.add(v[q], __fsub_rn(v[q], it.ref));
+                store([&](int q) {
+                    const float u = __fsub_rn(v[q], it.ref);
+                    if ((q + 1) * tile::THREADS <= G::ELEMS || threadIdx.x + q * tile::THREADS < G::ELEMS) check.add(v[q], u);
+                    return u;
+                });
             } else {
                 walk([&](int q, bool ok, int64_t) {
                     if (ok) check.add(v[q], __fsub_rn(v[q], it.ref));
                 });
+                store([&](int q) { return __fsub_rn(v[q], it.ref); });
             }
             it.sums = check.sums<P, R>(it.ref, nsteps);
+            if (it.sums) return it;
+            it.ref = 0.0f;
         }
-        if (!it.sums) it.ref = 0.0f;
-        store([&](int q) { return __fsub_rn(v[q], it.ref); });
+        store([&](int q) { return v[q]; });
     } else {
         store([&](int q) { return v[q]; });
     }

@@ -2393,8 +2393,10 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
             // at the end. `sums` applications fit the FP32 sum; it then goes to an integer.
             // The in += 1 of the thread's own points from the values its sums have just read, the halo beside
             // them; a pass over the whole tile where the extra registers cost more (n=8192, whole runs,
-            // us per application: star R=1 47 to 43, R=2 51 to 48; launches of eight, R=5 85 to 88).
-            constexpr bool FUSED_ADVANCE = P == STAR && R <= 2;
+            // us per application: star R=1 47 to 43, R=2 51 to 48; launches of eight, R=5 85 to 88; whole
+            // runs of 50 of the star grids of a batch of 256, which are evaluated in calls: 12.98 ms with it,
+            // 10.84 without).
+            constexpr bool FUSED_ADVANCE = P == STAR && R <= 2 && OUT_SRC != OUT_HBM;
             float a[ROWS][CPT] = {};
             int acc[ROWS][CPT] = {};
             int held = 0;
