@@ -18,7 +18,9 @@
  *     any 8-byte-aligned pointer works). The library allocates only where an entry point says so.
  *   - dtype PRK_FP64: in, in_next, out are double[n*n].
  *     dtype PRK_FP32C: in, in_next are float[n*n]; out is float[2*n*n], interleaved (hi, lo) pairs
- *     whose unevaluated sum hi+lo is the value (a compensated two-float accumulator).
+ *     whose unevaluated sum hi+lo is the value (a compensated two-float accumulator). Where the
+ *     exact result is no such pair, its last bits may differ with the launch depth, with the buffers'
+ *     alignment and between batched and single runs; FP64 results do not.
  *   - stream is a cudaStream_t passed as void* (NULL = the legacy default stream). Calls are
  *     stream-ordered and asynchronous unless stated otherwise. Calls on one stream from one host
  *     thread at a time.

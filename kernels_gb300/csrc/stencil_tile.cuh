@@ -21,12 +21,16 @@
 // (`depth`, any count): a whole run in one launch per tile, as the host-buffer path uses it on
 // bands of rows. STEPS = OPERATOR is the reference operator alone: out += S(in), no in_next.
 //
-// Evaluation modes:
-//   FP64, strict   every point in the reference order with binary64 instructions (bit-exact)
-//   FP64, exact    power-of-two stencils on a certified tile: integer evaluation with identical
-//                  bits (prk_fixed.cuh), falling back to strict per tile
-//   FP32C          paired antisymmetric differences from register row segments, summed per weight
-//                  group, split weights, TwoSum, two-float out (prk_arith.cuh)
+// Evaluation, chosen per tile from its values; FP64 gives the bits of the reference's order on every route:
+//   FP64, star R=1,2 and grid R=1   whole numbers: FP32 or integer arithmetic (prk_fixed.cuh); else binary64,
+//                  the power-of-two products joined to the adds
+//   FP64, the others   whole numbers of a small range: products from tables, the chain in fixed point (the
+//                  64-bit narrow form, else 96 bits); other whole numbers: products on the integer pipes;
+//                  reals: products shared between taps or joined to the adds; else every product and add
+//                  in binary64
+//   FP32C          whole numbers near one another: the taps times the weights' common denominator, exact in
+//                  FP32 (the integer route); else paired differences summed per weight group (the operator
+//                  form: one product per tap), split weights, TwoSum, two-float out (prk_arith.cuh)
 #pragma once
 
 #include <cuda.h>
@@ -62,9 +66,9 @@ constexpr int TH_DEFAULT = 32;
 constexpr int TH_TALL = 64;
 // STEPS of the operator form: one application of out += S(in), in untouched and no in_next. It takes
 // the same tiles and routes as the fused form and stores no in_next, so a power-of-two stencil moves 24
-// bytes per point at the copy rate: at n=8192, FP64, star R=2 2049 us on the generic kernels, 232 us
-// here (6.9 TB/s); grid R=4 18273 against 4044 us; FP32C star R=2 369 against 196 us, grid R=5 1677
-// against 599 us.
+// bytes per point at the copy rate: at n=8192, FP64, star R=2 2049 us on the generic kernels, 229 us
+// here (7.0 TB/s); grid R=4 18273 against 2134 us; FP32C star R=2 369 against 193 us, grid R=5 1677
+// against 365 us (reals: 1571).
 constexpr int OPERATOR = -1;
 constexpr bool one_application(int steps) { return steps == 1 || steps == OPERATOR; }
 // Deepest run-time depth for which the FP32 route holds: 15 * (2^20 + 65536) < 2^24.
@@ -353,8 +357,9 @@ __device__ __forceinline__ void fp32c_taps(const float* s, int ld, float (&sh)[C
 // partial sums small; in += 1 advances u. A thread's rows share every row segment it reads.
 // Bound by the FMA pipe (grid R >= 3) and by shared memory (about 28 bytes per point and application);
 // the group sums were bound by FP32 issue (star R=4, eight applications: FMA pipe 68%, issue 78%). At
-// n=8192, us per application of whole runs of 16, before and after: star R=2 87 to 51, star R=4 138 to
-// 61, star R=5 171 to 78, grid R=3 262 to 100, grid R=5 502 to 222; one application, grid R=5 591 to 420.
+// n=8192, us per application of whole runs of 16, group sums and this route: star R=2 87 and 48, star R=4
+// 138 and 61, star R=5 171 and 78, grid R=3 262 and 98, grid R=5 502 and 227; one application, grid R=5 589
+// and 374. Tiles off the route run as fast as without it (their loops share no registers with it).
 
 __host__ __device__ constexpr int gcd_of(int a, int b) { return b == 0 ? a : gcd_of(b, a % b); }
 
@@ -766,9 +771,6 @@ __device__ __forceinline__ bool out_units(uint64_t b, int shift, int32_t& V)
     return ok;
 }
 
-__device__ __forceinline__ uint64_t from_fixed_any(int64_t x, int unit) { return fx::from_fixed(x, unit); }
-__device__ __forceinline__ uint64_t from_fixed_any(int32_t x, int unit) { return from_fixed32(x, unit); }
-
 __device__ __forceinline__ double as_dbl(uint64_t b) { return __longlong_as_double(static_cast<long long>(b)); }
 __device__ __forceinline__ uint64_t as_bits(double d) { return static_cast<uint64_t>(__double_as_longlong(d)); }
 
@@ -1056,8 +1058,8 @@ static_assert(strict_taps_ok<STAR, 3>() && strict_taps_ok<STAR, 4>() && strict_t
               "strict tap groups");
 
 // Sixteenths of each chain that run in fixed point in the 96-bit form (the rest on the binary64 pipe),
-// per stencil and form (ONE: one application per launch; else several), as measured at n=16384 when
-// every tile took this form: star R=3, 4 11/16 and R=5 12/16 at one application, 14/16 and 13/16 at
+// per stencil and form (ONE: one application per launch; else several), as measured at n=16384 on tiles
+// that all took this form: star R=3, 4 11/16 and R=5 12/16 at one application, 14/16 and 13/16 at
 // several; grid R=2 11/16, R=3 12/16, R=4 13/16, R=5 15/16 at one, 12/16, 12/16, 14/16 and 13/16 at
 // several.
 template <int P, int R, bool ONE>
@@ -2655,8 +2657,7 @@ __device__ __forceinline__ void process_tile(unsigned char* stage, int* s_red, i
 
 // Register budget: the single-application kernels keep as many tiles resident as shared memory
 // allows, so that every SM has enough loads in flight; the multi-application kernels hold `out` in
-// registers and run at most four tiles per SM. The strict FP64 form is bound by the binary64 pipe
-// and gets the registers its unrolled tap sequence wants.
+// registers and run at most four tiles per SM.
 template <int P, int R, int DT, int STEPS, int TH_>
 constexpr int min_blocks()
 {

@@ -28,8 +28,7 @@ struct Smem {
     static_assert(BYTES <= tile::SMEM_PER_CTA_MAX, "the tile and its tables must fit in shared memory");
 };
 
-// Resident CTAs per SM the register budget is cut for: the TMA kernel's (three tiles per SM for the
-// table route), except for the FP64 power-of-two stencils at one application, whose out words are
+// Resident CTAs per SM the register budget is cut for: the TMA kernel's, except for the FP64 power-of-two stencils at one application, whose out words are
 // all requested ahead (tile::OUT_HBM_AHEAD) and which hold them in the registers of five CTAs per SM
 // rather than spilling at six (n=16383, star R=2: 3585 GFLOP/s against 3449 without the early
 // requests).
