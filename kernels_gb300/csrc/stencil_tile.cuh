@@ -1156,10 +1156,10 @@ __device__ __forceinline__ bool table_row_active(bool has_out, int64_t gi, int64
 // A tap is a loop iteration over eight points of a thread, which share its constants and descriptor, so
 // the code stays small at 110 taps; the tile holds table offsets instead of values, so a point's two
 // reads need no address arithmetic between them. What bounds it (ncu, grid R=5, n=8192, four
-// applications): shared memory 92% of its wavefronts (one for the offset, two for the product, per 32
-// points and tap) and the integer ALU 77%, 11.5 instructions per point and tap. At n=8192, us per
-// application, against the 96-bit form for every tile: one per launch, star R=3 925 to 648, grid R=2
-// 1296 to 849, grid R=5 6389 to 3143; whole runs of 16, star R=3 678 to 428, grid R=5 5342 to 2901.
+// applications): shared memory 86% of its wavefronts (one for the offset, two for the product, per 32
+// points and tap) and the integer ALU 79%, 12.3 instructions per point and tap. At n=8192, us per
+// application, against the 96-bit form for every tile: one per launch, star R=3 925 to 663, grid R=2
+// 1296 to 851, grid R=5 6389 to 3137; whole runs of 16, star R=3 678 to 426, grid R=5 5342 to 2894.
 // Slower: two products prefetched a tap ahead (grid R=2 888 and 722 at 24 warps), indices of four rows
 // packed in a word (grid R=5 3106: fewer wavefronts, more ALU instructions), the tie found through a
 // carry of the lowest kept bit (7 instructions, 3088).
